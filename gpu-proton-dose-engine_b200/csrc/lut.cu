@@ -112,31 +112,13 @@ __device__ double interp(double x, const double* xp, const double* fp, int n, do
     return slope * (x - xp[lo]) + fp[lo];
 }
 
-// numpy.interp where xp = linspace(a, b, n) is generated on the fly.
-__device__ double interp_lin(double x, double a, double b, int n, const double* fp, double left,
-                             double right) {
-    if (x < a) return left;
-    if (x > b) return right;
-    if (x == b) return fp[n - 1];
-    int lo = 0, hi = n - 1;
-    while (hi - lo > 1) {
-        int mid = (lo + hi) >> 1;
-        if (lin(a, b, n, mid) <= x) lo = mid; else hi = mid;
-    }
-    double x0 = lin(a, b, n, lo);
-    if (x0 == x) return fp[lo];
-    double x1 = lin(a, b, n, lo + 1);
-    double slope = (fp[lo + 1] - fp[lo]) / (x1 - x0);
-    return slope * (x - x0) + fp[lo];
-}
-
 // numpy.linspace(a, b, n)[k] with its step (b - a) / (n - 1) passed in: the same value as lin().
 __device__ __forceinline__ double lin_s(double a, double b, int n, int k, double step) {
     if (k == n - 1) return b;
     return (double)k * step + a;
 }
 
-// The interval of x on linspace(a, b, n) that interp_lin's binary search finds, for a <= x <= b:
+// The interval of x on linspace(a, b, n) that np.interp's search finds, for a <= x <= b:
 // estimated from x * (1 / step) and corrected against the grid points themselves, whose values
 // fk * step + a (fk = (double)lo kept in step with lo -- integers below 2^53, so fk +- 1 is
 // exact) are those lin_s computes.  lo and its grid point x0 on return; x == b gives lo = n - 1,
@@ -208,24 +190,29 @@ __global__ void csda_kernel(const double* in, double* out, int n, int inverse) {
 // CSDA range +fd_step and -fd_step.
 struct LayerScal {
     double e0, r0, sig_r, zmax, h;
+    double step, inv;    // zmax / (n_idd - 1), the curve grid's step, and its reciprocal
     int conv_k;
-    int pad_;
+    int last;            // last bin that can hold dose
 };
 
 struct LutDims {
     int n_layers, nvar, nz, n_idd, n_fe;
     double fe_lo, fe_hi;      // Fermi-Eyges fine grid end points
+    double fe_step, fe_inv;   // its step and the step's reciprocal
     double fd_step;
 };
 
-// Setup of one (layer, variant): energy, range, sigma_R (physics.py:154-174, 310-322),
-// the binned CSDA dose (physics.py:362-370), the Gaussian kernel table and the local
-// scattering power on the Fermi-Eyges fine grid (physics.py:259-264).
-__global__ void layer_setup_kernel(pbd_lut_spec spec, LutDims dm, const double* energies,
-                                   const double* shift, LayerScal* scal, double* binned,
-                                   double* ker, double* t_fe) {
+// Scalars of one (layer, variant) per block: energy, range and sigma_R (physics.py:154-174,
+// 310-322).  4000 stopping powers per block, FP64 log and divisions: a block of 512 threads
+// keeps the FP64 pipe of its SM busy (with the fills below in the same 256-thread block, one
+// block per (layer, variant), the set-up took 78 us for 120 of them; now 14 + 15 us).
+constexpr int kScalThreads = 512;
+
+__global__ void __launch_bounds__(kScalThreads)
+layer_scal_kernel(pbd_lut_spec spec, LutDims dm, const double* energies, const double* shift,
+                  LayerScal* scal) {
     __shared__ double f_bohr[kBohrN];
-    __shared__ double red[256];
+    __shared__ double red[kScalThreads];
     const int lv = blockIdx.x;
     const int l = lv / dm.nvar, v = lv % dm.nvar;
     const double off = v == 0 ? 0.0 : (v == 1 ? dm.fd_step : -dm.fd_step);
@@ -262,6 +249,7 @@ __global__ void layer_setup_kernel(pbd_lut_spec spec, LutDims dm, const double* 
     } else if (spec.straggling_model == 1) {
         strag = spec.strag_coef * pow(r0, spec.strag_exp);
     }
+    if (threadIdx.x != 0) return;
     const double espr = kPowerP * spec.energy_spread * r0;
     const double sig_r = hypot(strag, espr);
     const int n = dm.n_idd;
@@ -272,39 +260,74 @@ __global__ void layer_setup_kernel(pbd_lut_spec spec, LutDims dm, const double* 
         double kf = ceil(16.0 * sig_r / h);
         kk = kf > (double)(n - 1) ? n - 1 : (int)kf;
     }
-    if (threadIdx.x == 0) {
-        LayerScal sc;
-        sc.e0 = e0; sc.r0 = r0; sc.sig_r = sig_r; sc.zmax = zmax; sc.h = h; sc.conv_k = kk;
-        sc.pad_ = 0;
-        scal[lv] = sc;
-    }
+    LayerScal sc;
+    sc.e0 = e0; sc.r0 = r0; sc.sig_r = sig_r; sc.zmax = zmax; sc.h = h; sc.conv_k = kk;
+    sc.step = (zmax - 0.0) / (double)(n - 1);
+    sc.inv = 1.0 / sc.step;
+    // bin k holds dose only where its near edge k zmax / n lies before the range
+    const double kr0 = floor(r0 / (zmax / (double)n)) + 1.0;
+    sc.last = kr0 < (double)(n - 1) ? (int)kr0 : n - 1;
+    scal[lv] = sc;
+}
+
+// The arrays of one (layer, variant): the binned CSDA dose (physics.py:362-370), the Gaussian
+// kernel table, and T h of the Fermi-Eyges grid -- the local scattering power (physics.py:
+// 259-264) times h = numpy.gradient of the grid.  Block (x: layer and variant, y: a share of
+// the entries); one range-table search per bin edge, shared through shared memory by the two
+// bins that meet there.  t_fe may be null (depth curves only).
+constexpr int kFillThreads = 256;
+constexpr int kFillBins = 1024;     // bins per block
+
+__device__ __forceinline__ double fe_h(const LutDims& dm, int j) {
+    const int n = dm.n_fe;
+    if (j == 0) return lin(dm.fe_lo, dm.fe_hi, n, 1) - lin(dm.fe_lo, dm.fe_hi, n, 0);
+    if (j == n - 1) return lin(dm.fe_lo, dm.fe_hi, n, n - 1) - lin(dm.fe_lo, dm.fe_hi, n, n - 2);
+    return (lin(dm.fe_lo, dm.fe_hi, n, j + 1) - lin(dm.fe_lo, dm.fe_hi, n, j - 1)) / 2.0;
+}
+
+__global__ void __launch_bounds__(kFillThreads)
+layer_fill_kernel(pbd_lut_spec spec, LutDims dm, const LayerScal* __restrict__ scal,
+                  double* __restrict__ binned, double* __restrict__ ker,
+                  double* __restrict__ t_fe) {
+    __shared__ double s_e[kFillBins + 1];
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // the scalars of this call
+    const int lv = blockIdx.x, n = dm.n_idd;
+    const LayerScal sc = scal[lv];
+    const double r0 = sc.r0, zmax = sc.zmax, h = sc.h;
     double* bin = binned + (size_t)lv * n;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        double zf = lin(0.0, zmax, n, k);
-        double ea = lin(0.0, zmax, n + 1, k);
-        double eb = lin(0.0, zmax, n + 1, k + 1);
-        double ena = ea < r0 ? energy_at_range(fmax(r0 - ea, 0.0)) : 0.0;
-        double enb = eb < r0 ? energy_at_range(fmax(r0 - eb, 0.0)) : 0.0;
-        double fl = exp(-zf / spec.atten_len);
-        bin[k] = fl * (ena - enb) / h;
-    }
-    if (sig_r > 0.0) {
-        double* kr = ker + (size_t)lv * n;
-        const double c = kInvSqrt2Pi / sig_r;
-        for (int k = threadIdx.x; k <= kk; k += blockDim.x) {
-            double t = (double)k * h;
-            kr[k] = h * (c * exp(-(t * t) / (2.0 * sig_r * sig_r)));
+    for (int k0 = blockIdx.y * kFillBins; k0 < n; k0 += gridDim.y * kFillBins) {
+        const int nb = min(kFillBins, n - k0);
+        __syncthreads();
+        for (int q = threadIdx.x; q <= nb; q += kFillThreads) {
+            const double ea = lin(0.0, zmax, n + 1, k0 + q);
+            s_e[q] = ea < r0 ? energy_at_range(fmax(r0 - ea, 0.0)) : 0.0;
+        }
+        __syncthreads();
+        for (int q = threadIdx.x; q < nb; q += kFillThreads) {
+            const double zf = lin(0.0, zmax, n, k0 + q);
+            const double fl = exp(-zf / spec.atten_len);
+            bin[k0 + q] = fl * (s_e[q] - s_e[q + 1]) / h;
         }
     }
+    const int t0 = blockIdx.y * kFillThreads + threadIdx.x, stride = gridDim.y * kFillThreads;
+    if (sc.sig_r > 0.0) {
+        double* kr = ker + (size_t)lv * n;
+        const double c = kInvSqrt2Pi / sc.sig_r;
+        for (int k = t0; k <= sc.conv_k; k += stride) {
+            double t = (double)k * h;
+            kr[k] = h * (c * exp(-(t * t) / (2.0 * sc.sig_r * sc.sig_r)));
+        }
+    }
+    if (t_fe == nullptr) return;
     double* tf = t_fe + (size_t)lv * dm.n_fe;
-    for (int i = threadIdx.x; i < dm.n_fe; i += blockDim.x) {
+    for (int i = t0; i < dm.n_fe; i += stride) {
         double zf = lin(dm.fe_lo, dm.fe_hi, dm.n_fe, i);
         double t = 0.0;
         if (zf < r0) {
             double el = energy_at_range(fmax(r0 - zf, 0.0));
             t = highland_local(fmax(el, 1e-3));
         }
-        tf[i] = t;
+        tf[i] = t * fe_h(dm, i);
     }
 }
 
@@ -378,70 +401,152 @@ conv_kernel(LutDims dm, const LayerScal* scal, const double* binned, const doubl
         if (i0 + b < n) out[i0 + b] = acc[b];
 }
 
-// Fermi-Eyges direct scattering integral B(zf_i) = sum_{j<i} (zf_i - zf_j)^2 T_j h_j,
-// physics.py:266-270, with h = numpy.gradient(zf).
-__device__ __forceinline__ double fe_h(const LutDims& dm, int j) {
+// The tables at the requested depths.  A depth needs the smoothed curve at two points of its
+// fine grid (np.interp's interval) and the scattering integral at two points of its own, so only
+// those are formed, straight from the bins and from T h: 2 nz sums of 2 K + 1 products instead
+// of n (the whole 6000-point convolution, 325 us for 120 (layer, variant) pairs at 128 depths)
+// and 2 nz instead of n_fe for the integral (120 us); both together take 53 us, bound by the
+// loads of the bins and kernel values through L1.
+//
+// One warp per (layer, variant, depth): the lanes stride over the bins (coalesced; the
+// windows of a block's neighbouring depths overlap, so they come from L1) and their sums are
+// added by a butterfly.  A block holds kEvalDepths depths of one layer with all its
+// variants, which combine into the range derivatives.
+//
+// With `smooth` given (2 nz points would cost more than the whole curve, see lut_build) the
+// curve is read instead of summed.
+constexpr int kEvalDepths = 8;
+
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// smooth[n0] and smooth[n0 + 1] of the straggling convolution (see conv_kernel): sums over the
+// bins |n - m| <= K.  Bins past the range are zero and are not read; for a depth before the
+// range, where the curve is of the peak's order, neither are bins more than 9 sigma_R away, whose
+// weights (< 3e-18 of the largest) lie below the sum's last bit.  Past the range, where those
+// weights are all there is, the window is the whole one.
+__device__ __forceinline__ void conv_two(const LayerScal& sc, int n, const double* __restrict__ bin,
+                                         const double* __restrict__ kr, int n0, int lane,
+                                         double& f0, double& f1) {
+    if (sc.sig_r <= 0.0) {
+        f0 = bin[n0];
+        f1 = n0 + 1 < n ? bin[n0 + 1] : 0.0;
+        return;
+    }
+    int K = sc.conv_k;
+    if (n0 < sc.last) {
+        const double k9 = ceil(9.0 * sc.sig_r * sc.inv) + 1.0;
+        K = k9 < (double)K ? (int)k9 : K;
+    }
+    const int m0 = max(0, n0 - K), m1 = min(sc.last, n0 + 1 + K);
+    double a0 = 0.0, a1 = 0.0;
+#pragma unroll 4
+    for (int m = m0 + lane; m <= m1; m += 32) {
+        const double b = __ldg(bin + m);
+        const int d0 = abs(n0 - m), d1 = abs(n0 + 1 - m);
+        a0 = __fma_rn(b, d0 <= K ? __ldg(kr + d0) : 0.0, a0);
+        a1 = __fma_rn(b, d1 <= K ? __ldg(kr + d1) : 0.0, a1);
+    }
+    f0 = warp_sum(a0);
+    f1 = warp_sum(a1);
+}
+
+// Fermi-Eyges direct scattering integral B(zf_i) = sum_{j<i} (zf_i - zf_j)^2 T_j h_j
+// (physics.py:266-270) at the grid points i0 and i0 + 1.
+__device__ __forceinline__ void fe_two(const LutDims& dm, const double* __restrict__ th, int i0,
+                                       int lane, double& b0, double& b1) {
     const int n = dm.n_fe;
-    if (j == 0) return lin(dm.fe_lo, dm.fe_hi, n, 1) - lin(dm.fe_lo, dm.fe_hi, n, 0);
-    if (j == n - 1) return lin(dm.fe_lo, dm.fe_hi, n, n - 1) - lin(dm.fe_lo, dm.fe_hi, n, n - 2);
-    return (lin(dm.fe_lo, dm.fe_hi, n, j + 1) - lin(dm.fe_lo, dm.fe_hi, n, j - 1)) / 2.0;
-}
-
-__global__ void fe_grid_kernel(LutDims dm, double* zf, double* hf) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < dm.n_fe; i += gridDim.x * blockDim.x) {
-        zf[i] = lin(dm.fe_lo, dm.fe_hi, dm.n_fe, i);
-        hf[i] = fe_h(dm, i);
+    const double step = dm.fe_step;
+    const double z0 = lin_s(dm.fe_lo, dm.fe_hi, n, i0, step);
+    const double z1 = lin_s(dm.fe_lo, dm.fe_hi, n, min(i0 + 1, n - 1), step);
+    double a0 = 0.0, a1 = 0.0;
+#pragma unroll 4
+    for (int j = lane; j <= i0; j += 32) {       // j = i0 adds 0 to b0 (and i0 = n - 1 uses b0 only)
+        const double zj = (double)j * step + dm.fe_lo, t = __ldg(th + j);
+        const double d0 = j < i0 ? z0 - zj : 0.0, d1 = z1 - zj;
+        a0 += d0 * d0 * t;
+        a1 += d1 * d1 * t;
     }
+    b0 = warp_sum(a0);
+    b1 = warp_sum(a1);
 }
 
-__global__ void fe_b_kernel(LutDims dm, const double* zf, const double* hf, const double* t_fe,
-                            double* b_fe) {
-    const int lv = blockIdx.x;
-    const int i = blockIdx.y * blockDim.x + threadIdx.x;
-    if (i >= dm.n_fe) return;
-    const double* tf = t_fe + (size_t)lv * dm.n_fe;
-    const double zi = zf[i];
-    double acc = 0.0;
-    for (int j = 0; j < i; ++j) {
-        double d = zi - zf[j];
-        acc += d * d * tf[j] * hf[j];
-    }
-    b_fe[(size_t)lv * dm.n_fe + i] = acc;
-}
-
-// Tables at the requested depths, all variants of one layer per block; the variants
-// combine into the range derivatives.
-__global__ void lut_output_kernel(pbd_lut_spec spec, LutDims dm, const LayerScal* scal,
-                                  const double* smooth, const double* zf_fe, const double* b_fe,
-                                  double single_depth, double* idd, double* sigma,
-                                  double* didd, double* dsig) {
-    const int l = blockIdx.x;
-    for (int k = threadIdx.x; k < dm.nz; k += blockDim.x) {
-        double d = spec.depth_scale * (spec.z0 + (double)k * spec.dz);
-        double dz_eval = (dm.nz == 1 && !spec.anchor_surface) ? single_depth : d;
-        double out_i[3], out_s[3];
-        for (int v = 0; v < dm.nvar; ++v) {
-            const int lv = l * dm.nvar + v;
-            const LayerScal sc = scal[lv];
-            out_i[v] = interp_lin(d, 0.0, sc.zmax, dm.n_idd, smooth + (size_t)lv * dm.n_idd, 0.0,
-                                  0.0);
-            double b = 0.0;
-            if (!(spec.anchor_surface && d <= 0.0))
-                b = interp(dz_eval, zf_fe, b_fe + (size_t)lv * dm.n_fe, dm.n_fe,
-                           b_fe[(size_t)lv * dm.n_fe], b_fe[(size_t)lv * dm.n_fe + dm.n_fe - 1]);
-            double zp = dz_eval / spec.depth_scale;
-            double var = spec.sigma_x0 * spec.sigma_x0
-                       + 2.0 * spec.rho0 * spec.sigma_x0 * spec.sigma_theta0 * zp
-                       + spec.sigma_theta0 * spec.sigma_theta0 * (zp * zp)
-                       + b / (spec.depth_scale * spec.depth_scale);
-            out_s[v] = sqrt(fmax(var, 0.0));
+__global__ void __launch_bounds__(kEvalDepths * 3 * 32)
+lut_eval_kernel(pbd_lut_spec spec, LutDims dm, const LayerScal* __restrict__ scal,
+                const double* __restrict__ binned, const double* __restrict__ ker,
+                const double* __restrict__ smooth, const double* __restrict__ t_fe,
+                double single_depth, double* idd, double* sigma, double* didd, double* dsig) {
+    __shared__ double s_i[3][kEvalDepths], s_s[3][kEvalDepths];
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // the arrays of this call
+    const int nb = (dm.nz + kEvalDepths - 1) / kEvalDepths;      // blocks per layer
+    const int l = blockIdx.x / nb, k0 = (blockIdx.x - l * nb) * kEvalDepths;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int v = warp / kEvalDepths, kd = warp % kEvalDepths;
+    const int k = k0 + kd;
+    if (k < dm.nz) {
+        const int lv = l * dm.nvar + v;
+        const LayerScal sc = scal[lv];
+        const int n = dm.n_idd;
+        const double d = spec.depth_scale * (spec.z0 + (double)k * spec.dz);
+        const double dz_eval = (dm.nz == 1 && !spec.anchor_surface) ? single_depth : d;
+        // depth dose: np.interp on linspace(0, zmax, n), 0 outside
+        double out_i = 0.0;
+        if (!(d < 0.0 || d > sc.zmax)) {
+            int lo = 0;
+            double x0 = 0.0, f0, f1;
+            locate_lin(d, 0.0, sc.zmax, n, sc.step, sc.inv, lo, x0);
+            if (smooth) {
+                const double* fp = smooth + (size_t)lv * n;
+                f0 = fp[lo];
+                f1 = lo + 1 < n ? fp[lo + 1] : 0.0;
+            } else {
+                conv_two(sc, n, binned + (size_t)lv * n, ker + (size_t)lv * n, lo, lane, f0, f1);
+            }
+            if (x0 == d) {
+                out_i = f0;
+            } else {
+                const double x1 = lin_s(0.0, sc.zmax, n, lo + 1, sc.step);
+                out_i = (f1 - f0) / (x1 - x0) * (d - x0) + f0;
+            }
         }
-        const size_t o = (size_t)l * dm.nz + k;
-        idd[o] = out_i[0];
-        sigma[o] = out_s[0];
+        // lateral width: np.interp on the Fermi-Eyges grid, the end values outside
+        double b = 0.0;
+        if (!(spec.anchor_surface && d <= 0.0)) {
+            const int nf = dm.n_fe;
+            const double x = fmin(fmax(dz_eval, dm.fe_lo), dm.fe_hi);
+            int lo = 0;
+            double x0 = 0.0, b0, b1;
+            locate_lin(x, dm.fe_lo, dm.fe_hi, nf, dm.fe_step, dm.fe_inv, lo, x0);
+            fe_two(dm, t_fe + (size_t)lv * nf, lo, lane, b0, b1);
+            if (x0 == x) {
+                b = b0;
+            } else {
+                const double x1 = lin_s(dm.fe_lo, dm.fe_hi, nf, lo + 1, dm.fe_step);
+                b = (b1 - b0) / (x1 - x0) * (x - x0) + b0;
+            }
+        }
+        const double zp = dz_eval / spec.depth_scale;
+        const double var = spec.sigma_x0 * spec.sigma_x0
+                         + 2.0 * spec.rho0 * spec.sigma_x0 * spec.sigma_theta0 * zp
+                         + spec.sigma_theta0 * spec.sigma_theta0 * (zp * zp)
+                         + b / (spec.depth_scale * spec.depth_scale);
+        if (lane == 0) {
+            s_i[v][kd] = out_i;
+            s_s[v][kd] = sqrt(fmax(var, 0.0));
+        }
+    }
+    __syncthreads();
+    const int t = threadIdx.x, ko = k0 + t;
+    if (t < kEvalDepths && ko < dm.nz) {
+        const size_t o = (size_t)l * dm.nz + ko;
+        idd[o] = s_i[0][t];
+        sigma[o] = s_s[0][t];
         if (dm.nvar == 3) {
-            if (didd) didd[o] = (out_i[1] - out_i[2]) / (2.0 * dm.fd_step);
-            if (dsig) dsig[o] = (out_s[1] - out_s[2]) / (2.0 * dm.fd_step);
+            if (didd) didd[o] = (s_i[1][t] - s_i[2][t]) / (2.0 * dm.fd_step);
+            if (dsig) dsig[o] = (s_s[1][t] - s_s[2][t]) / (2.0 * dm.fd_step);
         }
     }
 }
@@ -593,7 +698,7 @@ __global__ void __launch_bounds__(kCmbThreads, 5) wed_combine_kernel(
                     const int i = tid + j * kCmbThreads;
                     if (i >= cnt || d[j] < 0.0 || d[j] > zm) continue;
                     const double2 pt = __ldg(lp + lo[j]);
-                    // interp_lin's value: fp[lo] on a grid point, else slope * (x - x0) + fp[lo]
+                    // np.interp's value: fp[lo] on a grid point, else slope * (x - x0) + fp[lo]
                     // with the slope np.interp rounds; the sum in layer order
                     const double idd = x0[j] == d[j] ? pt.x : pt.y * (d[j] - x0[j]) + pt.x;
                     if (idd == 0.0) continue;
@@ -705,7 +810,7 @@ __global__ void __launch_bounds__(256) wed_grad_maps_dr_kernel(
 
 // Curve points of the smoothed depth curves: {fp[k], slope_k} with slope_k = (fp[k+1] - fp[k])
 // / (x[k+1] - x[k]) on the grid linspace(0, zmax, n) -- the operands and the single rounding
-// of np.interp's slope (and of interp_lin) -- and 0 at the last point.  Value and slope share a
+// of np.interp's slope (and of lut_eval_kernel) -- and 0 at the last point.  Value and slope share a
 // 16-byte load in the combine, which needs no division per voxel.
 __global__ void wed_slope_kernel(LutDims dm, const LayerScal* scal, const double* smooth,
                                  double2* pts) {
@@ -875,8 +980,23 @@ int ensure_range_table(cudaStream_t st) {
 
 struct LutWs {
     LayerScal* scal;
-    double *binned, *ker, *smooth, *t_fe, *b_fe, *zf_fe, *hf_fe;
+    double *binned, *ker, *smooth, *t_fe;
 };
+
+// Scalars, then the arrays, of every (layer, variant); the fills start as the scalars' blocks
+// end (a programmatic dependent).  The first launch is an ordinary one: it must not start while
+// an earlier call on the stream still reads the workspace.
+int launch_layer_setup(const pbd_lut_spec& spec, const LutDims& dm, const double* energies,
+                       const double* shift, const LutWs& w, double* t_fe, cudaStream_t st) {
+    const int lvn = dm.n_layers * dm.nvar;
+    layer_scal_kernel<<<lvn, kScalThreads, 0, st>>>(spec, dm, energies, shift, w.scal);
+    PBD_LAUNCH_CHECK();
+    const int parts = std::min((dm.n_idd + kFillBins - 1) / kFillBins, 64);
+    PBD_TRY(launch_dependent(layer_fill_kernel, dim3(lvn, parts), dim3(kFillThreads), 0, st, spec,
+                             dm, (const LayerScal*)w.scal, w.binned, w.ker, t_fe));
+    count_launch(2);
+    return PBD_OK;
+}
 
 size_t carve_lut(Carve& c, LutWs& w, int n_layers, int nvar, int n_idd, int n_fe) {
     const size_t lv = (size_t)n_layers * nvar;
@@ -885,9 +1005,6 @@ size_t carve_lut(Carve& c, LutWs& w, int n_layers, int nvar, int n_idd, int n_fe
     w.ker = c.take<double>(lv * n_idd);
     w.smooth = c.take<double>(lv * n_idd);
     w.t_fe = c.take<double>(lv * n_fe);
-    w.b_fe = c.take<double>(lv * n_fe);
-    w.zf_fe = c.take<double>(n_fe);
-    w.hf_fe = c.take<double>(n_fe);
     return c.used;
 }
 
@@ -921,6 +1038,8 @@ int lut_build(const pbd_lut_spec* s, int n_layers, const double* energies, const
     dm.n_fe = fl.n_fine;
     dm.fe_lo = fl.lo;
     dm.fe_hi = fl.hi;
+    dm.fe_step = (fl.hi - fl.lo) / (double)(fl.n_fine - 1);
+    dm.fe_inv = 1.0 / dm.fe_step;
     dm.fd_step = s->fd_step;
     Carve c(ws);
     LutWs w;
@@ -928,21 +1047,28 @@ int lut_build(const pbd_lut_spec* s, int n_layers, const double* energies, const
     const int lvn = n_layers * dm.nvar;
 
     PBD_TRY(ensure_range_table(st));
-    fe_grid_kernel<<<(dm.n_fe + 255) / 256, 256, 0, st>>>(dm, w.zf_fe, w.hf_fe);
-    PBD_LAUNCH_CHECK();
-    layer_setup_kernel<<<lvn, 256, 0, st>>>(*s, dm, energies, shift, w.scal, w.binned, w.ker,
-                                            w.t_fe);
-    PBD_LAUNCH_CHECK();
-    conv_kernel<<<dim3(lvn, (dm.n_idd + kConvSeg - 1) / kConvSeg), kConvThreads, kConvSmem, st>>>(
-        dm, w.scal, w.binned, w.ker, w.smooth);
-    PBD_LAUNCH_CHECK();
-    fe_b_kernel<<<dim3(lvn, (dm.n_fe + 127) / 128), 128, 0, st>>>(dm, w.zf_fe, w.hf_fe, w.t_fe,
-                                                                  w.b_fe);
-    PBD_LAUNCH_CHECK();
-    lut_output_kernel<<<n_layers, 128, 0, st>>>(*s, dm, w.scal, w.smooth, w.zf_fe, w.b_fe,
-                                                 fl.single_depth, idd, sigma, didd, dsig);
-    PBD_LAUNCH_CHECK();
-    count_launch(5);
+    PBD_TRY(launch_layer_setup(*s, dm, energies, shift, w, w.t_fe, st));
+    // A depth's two points cost a warp 2 (2 K + 1) products at about a quarter of the rate of
+    // the whole curve's blocked convolution, which forms n of them.  Measured (40 layers x 3
+    // variants, n = 6000), points against the whole curve: 375 depths 171 / 435 us, 1024 depths
+    // 553 / 706, 1500 depths 927 / 1002; the points grow with the depths, so the curve from there.
+    const double* smooth = nullptr;
+    if (4LL * dm.nz >= dm.n_idd) {
+        conv_kernel<<<dim3(lvn, (dm.n_idd + kConvSeg - 1) / kConvSeg), kConvThreads, kConvSmem,
+                      st>>>(dm, w.scal, w.binned, w.ker, w.smooth);
+        PBD_LAUNCH_CHECK();
+        count_launch(1);
+        smooth = w.smooth;
+    }
+    const long long blocks = (long long)((dm.nz + kEvalDepths - 1) / kEvalDepths) * n_layers;
+    if (blocks > 2147483647LL) return PBD_ERR_UNSUPPORTED;
+    PBD_TRY(launch_dependent(lut_eval_kernel,
+                             dim3((unsigned)blocks),
+                             dim3(kEvalDepths * dm.nvar * 32), 0, st, *s, dm,
+                             (const LayerScal*)w.scal, (const double*)w.binned,
+                             (const double*)w.ker, smooth, (const double*)w.t_fe,
+                             fl.single_depth, idd, sigma, didd, dsig));
+    count_launch(1);
     return PBD_OK;
 }
 
@@ -978,6 +1104,8 @@ static int wed_dims(const pbd_lut_spec* s, int n_layers, const void* ws, size_t 
     dm.n_fe = fl.n_fine;
     dm.fe_lo = fl.lo;
     dm.fe_hi = fl.hi;
+    dm.fe_step = (fl.hi - fl.lo) / (double)(fl.n_fine - 1);
+    dm.fe_inv = 1.0 / dm.fe_step;
     dm.fd_step = 0.0;
     Carve c(const_cast<void*>(ws));
     carve_curves(c, w, pts, n_layers, dm.n_idd, dm.n_fe);
@@ -993,15 +1121,13 @@ int lut_wed_curves(const pbd_lut_spec* s, int n_layers, const double* energies,
     double2* pts = nullptr;
     PBD_TRY(wed_dims(s, n_layers, curves, curves_bytes, dm, w, pts));
     PBD_TRY(ensure_range_table(st));
-    layer_setup_kernel<<<n_layers, 256, 0, st>>>(*s, dm, energies, shift, w.scal, w.binned, w.ker,
-                                                 w.t_fe);
-    PBD_LAUNCH_CHECK();
+    PBD_TRY(launch_layer_setup(*s, dm, energies, shift, w, nullptr, st));
     conv_kernel<<<dim3(n_layers, (dm.n_idd + kConvSeg - 1) / kConvSeg), kConvThreads, kConvSmem, st>>>(
         dm, w.scal, w.binned, w.ker, w.smooth);
     PBD_LAUNCH_CHECK();
     wed_slope_kernel<<<n_layers, 256, 0, st>>>(dm, w.scal, w.smooth, pts);
     PBD_LAUNCH_CHECK();
-    count_launch(3);
+    count_launch(2);
     return PBD_OK;
 }
 
