@@ -1227,11 +1227,12 @@ int pbd_adjoint_wed(const pbd_field* f, const pbd_lut_spec* spec, const void* cu
     if (!workspace || workspace_bytes < need) return PBD_ERR_WORKSPACE;
     PBD_TRY(carve_wed_adj(f, precision, 1, workspace, wc, &need));
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t nslice = (size_t)f->ny * f->nx, nvox = (size_t)f->nz * nslice;
+    const size_t nslice = (size_t)f->ny * f->nx;
     PBD_TRY(lut_wed_activity(spec, f->n_layers, curves, curves_bytes, wed, f->nz, nslice, wc.act,
                              s));
-    PBD_TRY(lut_wed_grad_maps(spec, f->n_layers, curves, curves_bytes, grad_dose, wed, nvox,
-                              wed_lateral_stride(f), wc.maps, s));
+    PBD_TRY(lut_wed_grad_maps(spec, f->n_layers, curves, curves_bytes, nullptr, nullptr, 0.0,
+                              grad_dose, wed, f->nz, nslice, wc.act, wed_lateral_stride(f),
+                              wc.maps, s));
     return wed_adjoint_jobs(f, wc, w, sigma, nullptr, grad_w, nullptr, precision, s);
 }
 
@@ -1265,17 +1266,15 @@ int pbd_adjoint_wed_range(const pbd_field* f, const pbd_lut_spec* spec, const vo
     PBD_TRY(carve_wed_adj(f, precision, 2, workspace, wc, &need));
     cudaStream_t s = (cudaStream_t)stream;
     const int L = f->n_layers;
-    const size_t nslice = (size_t)f->ny * f->nx, nvox = (size_t)f->nz * nslice;
+    const size_t nslice = (size_t)f->ny * f->nx;
     const size_t lstride = wed_lateral_stride(f);
     // set 0: g IDD_l(WED) on the nominal curves' active slices; set 1: g dIDD_l/dR(WED) on the
     // slices that either shifted curve reaches
     PBD_TRY(lut_wed_activity(spec, L, curves, curves_bytes, wed, f->nz, nslice, wc.act, s));
-    PBD_TRY(lut_wed_grad_maps(spec, L, curves, curves_bytes, grad_dose, wed, nvox, lstride,
-                              wc.maps, s));
     PBD_TRY(lut_wed_activity(spec, L, curves_p, curves_bytes, wed, f->nz, nslice,
                              wc.act + (size_t)L * f->nz, s, curves_m, curves_bytes));
-    PBD_TRY(lut_wed_grad_maps_dr(spec, L, curves_p, curves_bytes, curves_m, curves_bytes, h,
-                                 grad_dose, wed, nvox, lstride, wc.maps + (size_t)L * lstride, s));
+    PBD_TRY(lut_wed_grad_maps(spec, L, curves, curves_bytes, curves_p, curves_m, h, grad_dose, wed,
+                              f->nz, nslice, wc.act, lstride, wc.maps, s));
     return wed_adjoint_jobs(f, wc, w, sigma, dsigma_dr, grad_w, grad_range, precision, s);
 }
 

@@ -150,6 +150,43 @@ __device__ __forceinline__ void locate_lin(double x, double a, double b, int n, 
     x0_out = x0;
 }
 
+// locate_lin on linspace(0, zmax, n) for 0 <= x <= zmax (or NaN: some lo in range): the estimate
+// floor(x inv) by adding 1.5 2^52, whose sum's low word is the integer -- two FP64 additions
+// instead of two conversions at a quarter of their rate -- then the same correction.
+__device__ __forceinline__ void locate_curve(double x, double zmax, int n, double step, double inv,
+                                             int& lo_out, double& x0_out) {
+    constexpr double kMagic = 6755399441055744.0;
+    const double t = (x * inv - 0.5) + kMagic;
+    int lo = __double2loint(t);
+    double fk = t - kMagic;
+    if (lo < 0 || lo > n - 2) {
+        lo = lo < 0 ? 0 : n - 2;
+        fk = (double)lo;
+    }
+    double x0 = fk * step;
+    if (x0 > x && lo > 0) {
+        do {
+            --lo;
+            fk -= 1.0;
+            x0 = fk * step;
+        } while (lo > 0 && x0 > x);
+    } else {
+        while (lo < n - 2) {
+            const double x1 = lo + 1 == n - 1 ? zmax : (fk + 1.0) * step;
+            if (!(x1 <= x)) break;
+            ++lo;
+            fk += 1.0;
+            x0 = x1;
+        }
+    }
+    if (x == zmax) {
+        lo = n - 1;
+        x0 = zmax;
+    }
+    lo_out = lo;
+    x0_out = x0;
+}
+
 __device__ __forceinline__ double csda(double e) {
     return interp(e, g_etab, g_rtab, kTableN, g_rtab[0], g_rtab[kTableN - 1]);
 }
@@ -691,7 +728,7 @@ __global__ void __launch_bounds__(kCmbThreads, 5) wed_combine_kernel(
                     lo[j] = 0;
                     x0[j] = 0.0;
                     if (tid + j * kCmbThreads < cnt && !(d[j] < 0.0 || d[j] > zm))
-                        locate_lin(d[j], 0.0, zm, n, st, is, lo[j], x0[j]);
+                        locate_curve(d[j], zm, n, st, is, lo[j], x0[j]);
                 }
 #pragma unroll
                 for (int j = 0; j < kCmbPer; ++j) {
@@ -736,74 +773,112 @@ __global__ void wed_poison_kernel(float* dose, size_t nvox, const int* err, cons
         dose[v] = __int_as_float(0x7fc00000);
 }
 
-// The heterogeneous dose's dL/dD seen by layer l: maps[l * lstride + v] = IDD_l(WED[v]) *
-// grad[v] (FP64 product, rounded once to FP32), 0 outside the curve.  The adjoint of layer l
-// with this map and depth dose 1 on its active slices is dL/dW_l.  Every (layer, voxel) entry
-// is written.
-__global__ void __launch_bounds__(256) wed_grad_maps_kernel(LutDims dm, const LayerScal* scal,
-                                                            const double2* pts, const float* grad,
-                                                            const double* wed, size_t nvox,
-                                                            int n_layers, size_t lstride,
-                                                            float* maps) {
-    __shared__ double zmax[kWedLayers], stp[kWedLayers], istp[kWedLayers];
-    for (int l = threadIdx.x; l < n_layers && l < kWedLayers; l += blockDim.x) {
-        zmax[l] = scal[l].zmax;
-        stp[l] = (scal[l].zmax - 0.0) / (double)(dm.n_idd - 1);
-        istp[l] = 1.0 / stp[l];
-    }
-    __syncthreads();
-    const int n = dm.n_idd;
-    for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nvox;
-         v += (size_t)gridDim.x * blockDim.x) {
-        const double d = wed[v];
-        const double g = (double)grad[v];
-        for (int l = 0; l < n_layers; ++l) {
-            const double zm = l < kWedLayers ? zmax[l] : scal[l].zmax;
-            float out = 0.0f;
-            if (!(d < 0.0 || d > zm)) {
-                const double st = l < kWedLayers ? stp[l] : (zm - 0.0) / (double)(n - 1);
-                const double is = l < kWedLayers ? istp[l] : 1.0 / st;
-                int lo = 0;
-                double x0 = 0.0;
-                locate_lin(d, 0.0, zm, n, st, is, lo, x0);
-                const double2 pt = __ldg(pts + (size_t)l * n + lo);
-                const double idd = x0 == d ? pt.x : pt.y * (d - x0) + pt.x;
-                out = (float)(idd * g);
-            }
-            maps[(size_t)l * lstride + v] = out;
-        }
-    }
-}
-
-// Depth dose of a layer's curve at depth d (the curve's interval search and np.interp
-// semantics, as in wed_grad_maps_kernel): 0 outside [0, zmax].
-__device__ __forceinline__ double curve_at(const LayerScal& sc, const double2* pts, int n, double d) {
-    const double zm = sc.zmax;
-    if (d < 0.0 || d > zm) return 0.0;
-    const double st = (zm - 0.0) / (double)(n - 1), is = 1.0 / st;
+// Depth dose of a layer's curve {value, slope} at depth d (np.interp's interval and value, 0
+// outside [0, zmax]); scalars as in LayerScal.
+struct CurveScal {
+    double zmax, step, inv;
+};
+__device__ __forceinline__ double curve_at(const CurveScal& c, const double2* __restrict__ pts, int n,
+                                           double d) {
+    if (d < 0.0 || d > c.zmax) return 0.0;
     int lo = 0;
     double x0 = 0.0;
-    locate_lin(d, 0.0, zm, n, st, is, lo, x0);
+    locate_curve(d, c.zmax, n, c.step, c.inv, lo, x0);
     const double2 pt = __ldg(pts + lo);
     return x0 == d ? pt.x : pt.y * (d - x0) + pt.x;
 }
 
-// maps (L, lstride): dL/dD times the range derivative of each layer's depth dose at the WED,
+// The heterogeneous dose's dL/dD seen by layer l: maps[l * lstride + v] = IDD_l(WED[v]) *
+// grad[v] (FP64 product, rounded once to FP32), 0 outside the curve.  The adjoint of layer l
+// with this map and depth dose 1 on its active slices is dL/dW_l.  kRange: also, at maps +
+// set_stride, dL/dD times the range derivative of the layer's depth dose at the WED,
 // (IDD+_l(WED) - IDD-_l(WED)) / (2 h), from the curves at range shifts +h and -h (FP64 difference,
-// one FP32 rounding of the product).
-__global__ void __launch_bounds__(256) wed_grad_maps_dr_kernel(
-    LutDims dm, const LayerScal* scp, const double2* ptp, const LayerScal* scm,
-    const double2* ptm, const float* grad, const double* wed, size_t nvox, int n_layers,
-    size_t lstride, double inv2h, float* maps) {
-    const int n = dm.n_idd;
-    for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nvox;
-         v += (size_t)gridDim.x * blockDim.x) {
-        const double d = wed[v];
-        const double g = (double)grad[v];
-        for (int l = 0; l < n_layers; ++l) {
-            const double dp = curve_at(scp[l], ptp + (size_t)l * n, n, d);
-            const double dmn = curve_at(scm[l], ptm + (size_t)l * n, n, d);
-            maps[(size_t)l * lstride + v] = (float)((dp - dmn) * inv2h * g);
+// one FP32 rounding of the product).  Only slices that the layer's activity table (act, act +
+// act_stride) marks are written: the adjoint reads no other.
+//
+// One block per 512 voxels of a slice, two per thread, over the slice's active layers.  Bound by
+// FP64 issue: some 12 operations per curve, the interval located without integer conversions
+// (a quarter of the FP64 rate).  One pass for both sets reads the WED and dL/dD once, and about
+// half of the (layer, slice) pairs are inactive: 128^3 x 28 layers, both sets, 497 us as two
+// kernels over every pair with a division per curve, 240 us
+// now, half of it the gathers of the curve points through L1.
+constexpr int kMapThreads = 256, kMapPer = 2;
+constexpr int kMapLayers = 128;   // layers staged together
+
+template <bool kRange>
+__global__ void __launch_bounds__(kMapThreads) wed_grad_maps_kernel(
+    int n, const LayerScal* __restrict__ scal, const double2* __restrict__ pts,
+    const LayerScal* __restrict__ scp, const double2* __restrict__ ptp,
+    const LayerScal* __restrict__ scm, const double2* __restrict__ ptm,
+    const float* __restrict__ grad, const double* __restrict__ wed, size_t nslice, int nz,
+    int n_layers, const double* __restrict__ act, size_t act_stride, size_t lstride,
+    size_t set_stride, double inv2h, float* __restrict__ maps) {
+    __shared__ CurveScal s_c[kRange ? 3 : 1][kMapLayers];
+    __shared__ int s_l[kMapLayers];      // active layers of the batch: index, bit 30 / 31: set 0 / 1
+    __shared__ int s_n;
+    const size_t nb = (nslice + kMapThreads * kMapPer - 1) / (kMapThreads * kMapPer);
+    const int z = (int)(blockIdx.x / nb);
+    const size_t v0 = (blockIdx.x - z * nb) * (kMapThreads * kMapPer) + threadIdx.x;
+    double d[kMapPer], g[kMapPer];
+    float* out[kMapPer];
+    bool in[kMapPer];
+#pragma unroll
+    for (int q = 0; q < kMapPer; ++q) {
+        const size_t v = v0 + q * kMapThreads;
+        in[q] = v < nslice;
+        const size_t o = (size_t)z * nslice + (in[q] ? v : 0);
+        d[q] = wed[o];
+        g[q] = (double)grad[o];
+        out[q] = maps + o;
+    }
+    for (int l0 = 0; l0 < n_layers; l0 += kMapLayers) {
+        __syncthreads();
+        if (threadIdx.x < 32) {          // the batch's active layers, in layer order
+            int cnt = 0;
+            for (int b = 0; b < kMapLayers; b += 32) {
+                const int l = l0 + b + (int)threadIdx.x;
+                unsigned f = 0u;
+                if (l < n_layers) {
+                    if (act[(size_t)l * nz + z] != 0.0) f |= 1u << 30;
+                    if (kRange && act[act_stride + (size_t)l * nz + z] != 0.0) f |= 1u << 31;
+                }
+                const unsigned bal = __ballot_sync(0xffffffffu, f != 0u);
+                if (f) s_l[cnt + __popc(bal & ((1u << threadIdx.x) - 1u))] = (int)(f | (unsigned)l);
+                cnt += __popc(bal);
+            }
+            if (threadIdx.x == 0) s_n = cnt;
+        }
+        __syncthreads();
+        const int na = s_n;
+        for (int k = threadIdx.x; k < na; k += kMapThreads) {
+            const int l = s_l[k] & 0x3FFFFFFF;
+            s_c[0][k] = CurveScal{scal[l].zmax, scal[l].step, scal[l].inv};
+            if constexpr (kRange) {
+                s_c[1][k] = CurveScal{scp[l].zmax, scp[l].step, scp[l].inv};
+                s_c[2][k] = CurveScal{scm[l].zmax, scm[l].step, scm[l].inv};
+            }
+        }
+        __syncthreads();
+        for (int k = 0; k < na; ++k) {
+            const unsigned f = (unsigned)s_l[k];
+            const size_t l = f & 0x3FFFFFFFu;
+            if (f & (1u << 30)) {
+#pragma unroll
+                for (int q = 0; q < kMapPer; ++q) {
+                    const double idd = curve_at(s_c[0][k], pts + l * n, n, d[q]);
+                    if (in[q]) out[q][l * lstride] = (float)(idd * g[q]);
+                }
+            }
+            if constexpr (kRange) {
+                if (f & (1u << 31)) {
+#pragma unroll
+                    for (int q = 0; q < kMapPer; ++q) {
+                        const double dp = curve_at(s_c[1][k], ptp + l * n, n, d[q]);
+                        const double dm = curve_at(s_c[2][k], ptm + l * n, n, d[q]);
+                        if (in[q]) out[q][set_stride + l * lstride] = (float)((dp - dm) * inv2h * g[q]);
+                    }
+                }
+            }
         }
     }
 }
@@ -1189,41 +1264,31 @@ int lut_wed_combine(const pbd_lut_spec* s, int n_layers, const float* lateral, s
 }
 
 int lut_wed_grad_maps(const pbd_lut_spec* s, int n_layers, const void* curves,
-                      size_t curves_bytes, const float* grad, const double* wed, size_t nvox,
-                      size_t lstride, float* maps, cudaStream_t st) {
+                      size_t curves_bytes, const void* curves_p, const void* curves_m, double h,
+                      const float* grad, const double* wed, int nz, size_t nslice,
+                      const double* act, size_t lstride, float* maps, cudaStream_t st) {
     PBD_TRY(validate_spec(s, n_layers));
-    if (!grad || !wed || !maps) return PBD_ERR_NULL_ARG;
+    if (!grad || !wed || !maps || !act) return PBD_ERR_NULL_ARG;
+    const size_t nvox = (size_t)nz * nslice;
     if (lstride < nvox) return PBD_ERR_BAD_VALUE;
-    LutDims dm;
-    LutWs w;
-    double2* pts = nullptr;
+    const bool range = curves_p != nullptr;
+    if (range && (!curves_m || !(h > 0.0) || !isfinite(h))) return PBD_ERR_BAD_VALUE;
+    LutDims dm, dp, dn;
+    LutWs w, wp{}, wm{};
+    double2 *pts = nullptr, *pp = nullptr, *pm = nullptr;
     PBD_TRY(wed_dims(s, n_layers, curves, curves_bytes, dm, w, pts));
-    const int blocks = (int)std::min<size_t>((nvox + 255) / 256, (size_t)num_sms() * 8);
-    wed_grad_maps_kernel<<<std::max(blocks, 1), 256, 0, st>>>(dm, w.scal, pts, grad, wed, nvox,
-                                                              n_layers, lstride, maps);
-    PBD_LAUNCH_CHECK();
-    count_launch(1);
-    return PBD_OK;
-}
-
-int lut_wed_grad_maps_dr(const pbd_lut_spec* s, int n_layers, const void* curves_p,
-                         size_t curves_p_bytes, const void* curves_m, size_t curves_m_bytes,
-                         double h, const float* grad, const double* wed, size_t nvox,
-                         size_t lstride, float* maps, cudaStream_t st) {
-    PBD_TRY(validate_spec(s, n_layers));
-    if (!grad || !wed || !maps || !curves_p || !curves_m) return PBD_ERR_NULL_ARG;
-    if (lstride < nvox) return PBD_ERR_BAD_VALUE;
-    if (!(h > 0.0) || !isfinite(h)) return PBD_ERR_BAD_VALUE;
-    LutDims dp, dmm;
-    LutWs wp, wm;
-    double2* pp = nullptr;
-    double2* pm = nullptr;
-    PBD_TRY(wed_dims(s, n_layers, curves_p, curves_p_bytes, dp, wp, pp));
-    PBD_TRY(wed_dims(s, n_layers, curves_m, curves_m_bytes, dmm, wm, pm));
-    const int blocks = (int)std::min<size_t>((nvox + 255) / 256, (size_t)num_sms() * 8);
-    wed_grad_maps_dr_kernel<<<std::max(blocks, 1), 256, 0, st>>>(dp, wp.scal, pp, wm.scal, pm, grad,
-                                                                 wed, nvox, n_layers, lstride,
-                                                                 0.5 / h, maps);
+    if (range) {
+        PBD_TRY(wed_dims(s, n_layers, curves_p, curves_bytes, dp, wp, pp));
+        PBD_TRY(wed_dims(s, n_layers, curves_m, curves_bytes, dn, wm, pm));
+    }
+    const size_t per = (size_t)kMapThreads * kMapPer;
+    const size_t blocks = (nslice + per - 1) / per * (size_t)nz;
+    if (blocks > 2147483647u) return PBD_ERR_UNSUPPORTED;
+    const size_t act_stride = (size_t)n_layers * nz, set_stride = (size_t)n_layers * lstride;
+    const auto kernel = range ? wed_grad_maps_kernel<true> : wed_grad_maps_kernel<false>;
+    kernel<<<(unsigned)blocks, kMapThreads, 0, st>>>(
+        dm.n_idd, w.scal, pts, wp.scal, pp, wm.scal, pm, grad, wed, nslice, nz, n_layers, act,
+        act_stride, lstride, set_stride, range ? 0.5 / h : 0.0, maps);
     PBD_LAUNCH_CHECK();
     count_launch(1);
     return PBD_OK;

@@ -265,17 +265,14 @@ int lut_wed_activity(const pbd_lut_spec* s, int n_layers, const void* curves, si
 int lut_wed_combine(const pbd_lut_spec* s, int n_layers, const float* lateral, size_t lstride,
                     const double* wed, size_t nvox, float* dose, int* err, const int* err2,
                     const void* curves, size_t curves_bytes, cudaStream_t st);
-// maps (L, lstride): dL/dD times each layer's depth dose at the WED (the heterogeneous
-// adjoint's per-layer input).
+// maps (L, lstride): dL/dD times each layer's depth dose at the WED (the heterogeneous adjoint's
+// per-layer input), written on the slices that act (L, nz) marks.  With curves_p / curves_m (the
+// curves at range shifts +h and -h, of the size of `curves`) also a second set after the first,
+// dL/dD times (IDD+_l(WED) - IDD-_l(WED)) / (2 h), on the slices that act + L nz marks.
 int lut_wed_grad_maps(const pbd_lut_spec* s, int n_layers, const void* curves,
-                      size_t curves_bytes, const float* grad, const double* wed, size_t nvox,
-                      size_t lstride, float* maps, cudaStream_t st);
-// maps (L, lstride): dL/dD times (IDD+_l(WED) - IDD-_l(WED)) / (2 h), the curves built at range
-// shifts +h and -h (the heterogeneous range gradient's per-layer input).
-int lut_wed_grad_maps_dr(const pbd_lut_spec* s, int n_layers, const void* curves_p,
-                         size_t curves_p_bytes, const void* curves_m, size_t curves_m_bytes,
-                         double h, const float* grad, const double* wed, size_t nvox,
-                         size_t lstride, float* maps, cudaStream_t st);
+                      size_t curves_bytes, const void* curves_p, const void* curves_m, double h,
+                      const float* grad, const double* wed, int nz, size_t nslice,
+                      const double* act, size_t lstride, float* maps, cudaStream_t st);
 int lut_wed_raytrace(int nz, int ny, int nx, double oz, double dz, const float* rho, double* wed,
                      cudaStream_t st);
 
