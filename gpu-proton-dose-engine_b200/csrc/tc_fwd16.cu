@@ -34,6 +34,13 @@
 //    two D accumulators, stage 2 cross products into the unit's accumulator; each commits to
 //    the barriers that release its operands and publish its result.
 //
+// What bounds it: the math warps' instruction issue and fetch (the tensor pipe is 15 % busy).  Their
+// phases are rolled loops over 8-column chunks in packed FP32 pairs (fma.rn.f32x2: the same bits
+// in half the instructions), E1's TMEM loads included, which a rolled loop waits 55 cycles for;
+// the MMA loops increment their descriptors.  Unrolled and with E1's loads issued a phase early the
+// dose kernel of the 128^3 / 41 x 41 x 40 field took 70 us, now 57, of 200 x 200 x 256 / 61 x 61 x 60
+// 973, now 850; the doses are the same bits.
+//
 // Accumulation as in the TF32 forward: the large products of a step go to a fresh accumulator
 // that the math warps add in FP32 registers (the tensor core truncates when it accumulates),
 // the cross products (~2^-11 of them) stay in one accumulator per unit.
@@ -115,16 +122,19 @@ __device__ __forceinline__ uint32_t h2bits(__half2 h) { return *reinterpret_cast
 __device__ __forceinline__ float round11(float a) {
     return __uint_as_float((__float_as_uint(a) + 0x1000u) & 0xFFFFE000u);
 }
-__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
+__device__ __forceinline__ void split2(f32x2 v, uint32_t& hi, uint32_t& lo) {
+    float a, b, ra, rb;
+    upk(v, a, b);
     const float ha = round11(a), hb = round11(b);
     hi = h2bits(__floats2half2_rn(ha, hb));
-    lo = h2bits(__floats2half2_rn(a - ha, b - hb));
+    upk(fma2(pk(ha, hb), pk(-1.0f, -1.0f), v), ra, rb);
+    lo = h2bits(__floats2half2_rn(ra, rb));
 }
 
-__device__ __forceinline__ void split8(const float* v, uint4& hi, uint4& lo) {
+__device__ __forceinline__ void split8(const f32x2* v, uint4& hi, uint4& lo) {
     uint32_t h[4], l[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) split2(v[2 * q], v[2 * q + 1], h[q], l[q]);
+    for (int q = 0; q < 4; ++q) split2(v[q], h[q], l[q]);
     hi = make_uint4(h[0], h[1], h[2], h[3]);
     lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
@@ -217,7 +227,8 @@ __global__ void __launch_bounds__(256) pack_w16_kernel(const JobDev* __restrict_
             v[k] = (i < nsx && j < nsy) ? ldexpf(ws[j * nsx + i], e) : 0.f;
         }
         uint4 hi, lo;
-        split8(v, hi, lo);
+        const f32x2 v2[4] = {pk(v[0], v[1]), pk(v[2], v[3]), pk(v[4], v[5]), pk(v[6], v[7])};
+        split8(v2, hi, lo);
         *reinterpret_cast<uint4*>(out + (size_t)g * rows * 16 + (size_t)r * 16) = r < N1 ? hi : lo;
     }
     if (threadIdx.x == 0) {
@@ -423,13 +434,47 @@ __device__ __forceinline__ Bars make_bars(uint64_t* b) {
 }
 constexpr int kNumBars = 30;
 
+// Issue loops of one thread, rolled with incremented descriptors (straight-line code is fetched
+// anew for every step).
+__device__ __forceinline__ void issue1(uint32_t tb, uint32_t a, uint32_t alo, uint32_t w, uint32_t plW,
+                                       int N1, int steps, uint32_t id1w, uint32_t id1n) {
+    constexpr uint32_t plA = 128u * 16u;
+    uint64_t ah = tc::smem_desc(a, plA, 128), wd = tc::smem_desc(w, plW, 128);
+    const uint64_t to_lo = alo >> 4, incA = plA >> 3, incW = plW >> 3;
+    uint32_t acc = 0u;
+#pragma unroll 1
+    for (int st = 0; st < steps; ++st) {
+        tc::mma_bf16(tb + kColU, ah, wd, id1w, acc);
+        tc::mma_bf16(tb + kColU + (uint32_t)N1, ah + to_lo, wd, id1n, 1u);
+        acc = 1u;
+        ah += incA;
+        wd += incW;
+    }
+}
+__device__ __forceinline__ void issue2(uint32_t d, uint32_t a, uint32_t b, uint32_t lo, int steps,
+                                       uint32_t id2, uint32_t acc, bool cross) {
+    constexpr uint32_t pl = 128u * 16u;
+    uint64_t ad = tc::smem_desc(a, pl, 128), bd = tc::smem_desc(b, pl, 128);
+    const uint64_t to_lo = lo >> 4, inc = pl >> 3;
+#pragma unroll 1
+    for (int st = 0; st < steps; ++st) {
+        if (cross) {
+            tc::mma_bf16(d, ad, bd + to_lo, id2, acc);
+            tc::mma_bf16(d, ad + to_lo, bd, id2, 1u);
+        } else {
+            tc::mma_bf16(d, ad, bd, id2, acc);
+        }
+        acc = 1u;
+        ad += inc;
+        bd += inc;
+    }
+}
+
 __device__ __forceinline__ void mma_warp(const Params& P, uint32_t sbase, uint32_t tb, int role,
                                          const Step* ring, uint64_t* full, uint64_t* empty,
                                          const Bars& B) {
     const int lane = threadIdx.x & 31;
     const int K1 = P.K1, N1 = P.N1;
-    const uint32_t plA = 128u * 16u;                 // plane of a 128-row operand
-    const uint32_t plW = 2u * (uint32_t)N1 * 16u;    // plane of the spot map (2 N1 rows)
     const uint32_t aBytes1 = (uint32_t)K1 * 256u;    // one half (hi or lo) of a Gx buffer
     const uint32_t aBytes2 = (uint32_t)N1 * 256u;    // one half of a Gy / sU buffer
     const uint32_t id1w = tc::instr_desc(128, 2 * N1, 0u);
@@ -461,13 +506,7 @@ __device__ __forceinline__ void mma_warp(const Params& P, uint32_t sbase, uint32
                                        : sbase + P.oA1 + (uint32_t)ia * 2u * aBytes1;
                 const uint32_t alo = sym ? aBytes2 : aBytes1;
                 const uint32_t w = sbase + P.oW + (uint32_t)ws * P.img;
-                for (int st = 0; st < K1 / 16; ++st) {
-                    const uint32_t oa = (uint32_t)st * 2u * plA, ow = (uint32_t)st * 2u * plW;
-                    tc::mma_bf16(tb + kColU, tc::smem_desc(a + oa, plA, 128),
-                                 tc::smem_desc(w + ow, plW, 128), id1w, st > 0 ? 1u : 0u);
-                    tc::mma_bf16(tb + kColU + (uint32_t)N1, tc::smem_desc(a + alo + oa, plA, 128),
-                                 tc::smem_desc(w + ow, plW, 128), id1n, 1u);
-                }
+                issue1(tb, a, alo, w, 2u * (uint32_t)N1 * 16u, N1, K1 / 16, id1w, id1n);
                 tc::commit(B.uf);
                 tc::commit(&B.a1f[ia]);
                 tc::commit(&B.wempty[ws]);
@@ -488,19 +527,8 @@ __device__ __forceinline__ void mma_warp(const Params& P, uint32_t sbase, uint32
             if (lane == 0) {
                 const uint32_t a = sbase + P.oA2 + (uint32_t)ia * 2u * aBytes2;
                 const uint32_t b = sbase + P.oB2 + (uint32_t)ib * 2u * aBytes2;
-                for (int st = 0; st < N1 / 16; ++st) {
-                    const uint32_t o = (uint32_t)st * 2u * plA;
-                    if (role == 2) {
-                        tc::mma_bf16(tb + kColDb + (uint32_t)db * 128u, tc::smem_desc(a + o, plA, 128),
-                                     tc::smem_desc(b + o, plA, 128), id2, st > 0 ? 1u : 0u);
-                    } else {
-                        tc::mma_bf16(tb + kColDc, tc::smem_desc(a + o, plA, 128),
-                                     tc::smem_desc(b + aBytes2 + o, plA, 128), id2,
-                                     (first && st == 0) ? 0u : 1u);
-                        tc::mma_bf16(tb + kColDc, tc::smem_desc(a + aBytes2 + o, plA, 128),
-                                     tc::smem_desc(b + o, plA, 128), id2, 1u);
-                    }
-                }
+                issue2(role == 2 ? tb + kColDb + (uint32_t)db * 128u : tb + kColDc, a, b, aBytes2, N1 / 16,
+                       id2, role == 2 || first ? 0u : 1u, role == 3);
                 if (role == 2) tc::commit(&B.df[db]);
                 tc::commit(&B.a2f[ia]);
                 tc::commit(&B.b2f[ib]);
@@ -536,9 +564,9 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
     float4* tab = reinterpret_cast<float4*>(smem + P.oTab);
     constexpr int kMaxR = 64 / 16;                   // chunk pairs per thread (K <= 64)
 
-    float dsum[64];
+    f32x2 dsum[32];                                  // this lane's 64 columns, two per register pair
 #pragma unroll
-    for (int q = 0; q < 64; ++q) dsum[q] = 0.f;
+    for (int q = 0; q < 32; ++q) dsum[q] = 0ull;
     bool ok = true;
     int k = 0;         // ring reads
     int ng = 0;        // steps generated (G done)
@@ -564,20 +592,22 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
             } else {
 #pragma unroll
                 for (int q = 0; q < 64; q += 4) {
+                    float v[4];
+                    upk(dsum[q / 2], v[0], v[1]);
+                    upk(dsum[q / 2 + 1], v[2], v[3]);
                     if (vec) {
-                        *reinterpret_cast<float4*>(o + q) =
-                            make_float4(dsum[q], dsum[q + 1], dsum[q + 2], dsum[q + 3]);
+                        *reinterpret_cast<float4*>(o + q) = make_float4(v[0], v[1], v[2], v[3]);
                     } else {
 #pragma unroll
                         for (int r = 0; r < 4; ++r)
-                            if (xb + q + r < J.nx) o[q + r] = dsum[q + r];
+                            if (xb + q + r < J.nx) o[q + r] = v[r];
                     }
                 }
             }
         }
         if (!zero) {
 #pragma unroll
-            for (int q = 0; q < 64; ++q) dsum[q] = 0.f;
+            for (int q = 0; q < 32; ++q) dsum[q] = 0ull;
         }
     };
 
@@ -625,7 +655,7 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
                 }
             }
         }
-        const float a2 = st.a2;
+        const f32x2 na2 = pk(-st.a2, -st.a2), gs2 = pk(kGScale, kGScale);
         uint8_t* a2h = smem + P.oA2 + (uint32_t)ia2 * 2u * aBytes2;
         uint8_t* a1h = smem + P.oA1 + (uint32_t)ia * 2u * aBytes1;
         auto operand = [&](int tab0, int nc, uint8_t* dst, uint32_t lo_off) {
@@ -634,9 +664,13 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
                 if (r < nc) {
                     const float4 p = tab[(tab0 + 2 * r) * kMath + tid];
                     const float4 q4 = tab[(tab0 + 2 * r + 1) * kMath + tid];
-                    float v[8] = {p.x, p.y, p.z, p.w, q4.x, q4.y, q4.z, q4.w};
+                    f32x2 v[4] = {pk(p.x, p.y), pk(p.z, p.w), pk(q4.x, q4.y), pk(q4.z, q4.w)};
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) v[e] = ex2_approx(fmaf(-v[e], a2, kGScale));
+                    for (int e = 0; e < 4; ++e) {
+                        float x0, x1;
+                        upk(fma2(v[e], na2, gs2), x0, x1);
+                        v[e] = pk(ex2_approx(x0), ex2_approx(x1));
+                    }
                     uint4 hi, lo;
                     split8(v, hi, lo);
                     const uint32_t off = (uint32_t)(ghalf + 2 * r) * 2048u + (uint32_t)grow * 16u;
@@ -656,52 +690,40 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
         return true;
     };
 
-    // E1: U of step m from TMEM, times f1, split -> B2[m % nB2] (x rows, K = j).
-    // E1 in two parts: the TMEM loads of U are issued before the next step's G, which hides
-    // their latency, and waited for after it (G issues no TMEM load of its own).
+    // E1: U of step m from TMEM, times f1, split -> B2[m % nB2] (x rows, K = j), 8 columns at a time.
     const int ncol = N1 / 2, c0 = half * ncol;   // this warp's columns j: multiple of 8
-    uint32_t rb[4][8], rc[4][8];
-    auto e1_issue = [&](int m) -> bool {
+    auto e1 = [&](const Step& st, int m) -> bool {
+        const int ib = m % P.nB2;
         bool w = wait_bar(B.uf, (uint32_t)(m & 1), P.wait_ns);
+        if (m >= P.nB2) w = w && wait_bar(&B.b2f[ib], (uint32_t)(((m / P.nB2) - 1) & 1), P.wait_ns);
         if (!__all_sync(0xffffffffu, w)) return false;
         tc::fence_after_sync();
+        const f32x2 f2 = pk(st.f1, st.f1);
+        const uint32_t u = tb + kColU + lane_base + (uint32_t)c0;
+        uint8_t* bh = smem + P.oB2 + (uint32_t)ib * 2u * aBytes2 + (uint32_t)(c0 >> 3) * 2048u + (uint32_t)trow * 16u;
+#pragma unroll 1
+        for (int c = 0; c < ncol; c += 8, bh += 2048) {
+            uint32_t rb[8], rc[8];
+            tc::tmem_ld8(u + (uint32_t)c, rb);
+            tc::tmem_ld8(u + (uint32_t)(N1 + c), rc);
+            tc::tmem_wait_ld();
+            f32x2 v[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (q * 8 < ncol) {
-                tc::tmem_ld8(tb + kColU + lane_base + (uint32_t)(c0 + 8 * q), rb[q]);
-                tc::tmem_ld8(tb + kColU + lane_base + (uint32_t)(N1 + c0 + 8 * q), rc[q]);
-            }
+            for (int e = 0; e < 4; ++e)
+                v[e] = mul2(add2(pk(__uint_as_float(rb[2 * e]), __uint_as_float(rb[2 * e + 1])),
+                                 pk(__uint_as_float(rc[2 * e]), __uint_as_float(rc[2 * e + 1]))), f2);
+            uint4 hi, lo;
+            split8(v, hi, lo);
+            *reinterpret_cast<uint4*>(bh) = hi;
+            *reinterpret_cast<uint4*>(bh + aBytes2) = lo;
         }
-        return true;
-    };
-    auto e1 = [&](const Step& st, int m) -> bool {
-        bool w = true;
-        tc::tmem_wait_ld();
         tc::fence_before_sync();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(B.uu);
-        const int ib = m % P.nB2;
-        if (m >= P.nB2) w = wait_bar(&B.b2f[ib], (uint32_t)(((m / P.nB2) - 1) & 1), P.wait_ns);
-        if (!__all_sync(0xffffffffu, w)) return false;
-        uint8_t* bh = smem + P.oB2 + (uint32_t)ib * 2u * aBytes2;
-        const float f1 = st.f1;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (q * 8 < ncol) {
-                float v[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    v[e] = (__uint_as_float(rb[q][e]) + __uint_as_float(rc[q][e])) * f1;
-                uint4 hi, lo;
-                split8(v, hi, lo);
-                const uint32_t off = (uint32_t)((c0 >> 3) + q) * 2048u + (uint32_t)trow * 16u;
-                *reinterpret_cast<uint4*>(bh + off) = hi;
-                *reinterpret_cast<uint4*>(bh + aBytes2 + off) = lo;
-            }
-        }
         tc::fence_async_smem();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&B.b2r[ib]);
+        if (lane == 0) {
+            tc::mbar_arrive(B.uu);
+            tc::mbar_arrive(&B.b2r[ib]);
+        }
         return true;
     };
 
@@ -712,6 +734,7 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
         if (!__all_sync(0xffffffffu, w)) return false;
         tc::fence_after_sync();
         const float sc = __int_as_float((127 - st.kd) << 23);   // 2^-kd, exact (|kd| <= 114)
+        const f32x2 sc2 = pk(sc, sc);
         uint32_t r[4][16];
 #pragma unroll
         for (int c = 0; c < 4; ++c)
@@ -723,7 +746,8 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
 #pragma unroll
         for (int c = 0; c < 4; ++c)
 #pragma unroll
-            for (int q = 0; q < 16; ++q) dsum[c * 16 + q] = fmaf(__uint_as_float(r[c][q]), sc, dsum[c * 16 + q]);
+            for (int q = 0; q < 8; ++q)
+                dsum[c * 8 + q] = fma2(pk(__uint_as_float(r[c][2 * q]), __uint_as_float(r[c][2 * q + 1])), sc2, dsum[c * 8 + q]);
         if (st.flags & kLast) {
             w = wait_bar(B.cf, (uint32_t)(useg & 1), P.wait_ns);
             if (!__all_sync(0xffffffffu, w)) return false;
@@ -739,7 +763,8 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
 #pragma unroll
             for (int c = 0; c < 4; ++c)
 #pragma unroll
-                for (int q = 0; q < 16; ++q) dsum[c * 16 + q] = fmaf(__uint_as_float(r[c][q]), sc, dsum[c * 16 + q]);
+                for (int q = 0; q < 8; ++q)
+                    dsum[c * 8 + q] = fma2(pk(__uint_as_float(r[c][2 * q]), __uint_as_float(r[c][2 * q + 1])), sc2, dsum[c * 8 + q]);
             output(st, false);
         }
         return true;
@@ -774,16 +799,9 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
                 have = true;
             }
         }
-        if (p1) {
-            ok = e1_issue(i1);
-            if (!ok) break;
-        }
         if (have) {
             ok = gen(cur, ng);
-            if (!ok) {
-                tc::tmem_wait_ld();   // the E1 loads in flight land before the kernel leaves
-                break;
-            }
+            if (!ok) break;
         }
         if (p1) {
             ok = e1(s1, i1);
