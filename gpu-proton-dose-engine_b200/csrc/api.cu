@@ -241,7 +241,7 @@ int carve_ws(const pbd_field* f, bool fwd, bool adj, bool loss, int precision, v
     if (adj) {
         size_t pe = 0;
         int n1 = 0;
-        if (tc_adjoint_dims(precision, f, &n1) == PBD_OK) {
+        if (tc_adjoint_dims_tiled(precision, f, &n1) == PBD_OK) {
             // tensor-core adjoint: (slice, layer-chunk) units, one slot and the warps' dot
             // products per active (layer, slice)
             w.adj_tc = 1;

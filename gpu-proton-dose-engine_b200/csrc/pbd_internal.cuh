@@ -197,7 +197,10 @@ int launch_slice_schedule(JobDev* jobs_dev, FwdItem* items, int chunk, int n_job
 // pulled z-major; `partial` holds one (layer, slice) slot plane of nsy * nsx floats and the
 // warps' dot-product partials of every pair (tc_adjoint_slot_elems); counter[0] = unit
 // counter, counter[1] unused; `err` = the error word (cleared by the caller).
+// tc_adjoint_dims: one tile (nx, ny <= 128: the batched and heterogeneous calls);
+// tc_adjoint_dims_tiled: ny <= 256, any number of 128-column tiles (the single-field calls).
 int tc_adjoint_dims(int precision, const pbd_field* f, int* N1);
+int tc_adjoint_dims_tiled(int precision, const pbd_field* f, int* N1);
 // The calling thread's explicit adjoint item size (pbd_set_schedule), 0 when none is set.
 int schedule_adj_override();
 size_t tc_adjoint_slot_elems(const pbd_field* f);
