@@ -2,7 +2,7 @@
 //
 // D[z,y,x] = sum_l IDD_l(z) sum_j Gy[y,j] sum_i W_l[j,i] Gx[x,i]   (engines.py:191-197)
 //
-// Work item = (job, depth slice z, 128x128 lateral tile, chunk of <= C active layers).
+// Work item = (job, depth slice z, lateral tile of at most 128x128, chunk of <= C active layers).
 // For each active layer the CTA generates the Gaussian factors of that (layer, slice)
 // in shared memory (never stored in HBM), contracts
 //     U[j, x] = sum_i W'[j,i] Gx[x,i]      (W' = W * IDD / (2 pi sigma^2))
@@ -22,8 +22,26 @@ namespace {
 
 constexpr int NT = 256;
 constexpr int SC = kSpotChunk;                      // 64 spots per chunk
-constexpr int kFwdSmemFloats = 3 * SC * kTile + SC * SC;
-constexpr size_t kFwdSmemBytes = kFwdSmemFloats * sizeof(float);   // 112 KiB
+// shared memory of a 16 RY x 16 RX tile with spot chunks of sc (128 x 128, 64 spots: 112 KiB)
+constexpr size_t fwd_smem(int ry, int rx, int sc) {
+    return (size_t)(sc * 16 * (2 * rx + ry) + sc * SC) * sizeof(float);
+}
+
+// Tile sizes per axis, in units of 16 voxels.  An axis of n voxels is cut into ceil(n / 128) tiles of
+// equal size, rounded up to one of these: a 150 x 142 slice in four 80 x 80 tiles instead of four
+// 128 x 128 ones, of which two thirds were outside the grid.  The kernel is bound by FP32 FMA issue, so
+// its time follows the padded area: 150 x 142 x 160, 24 layers of 73 x 73 spots (cut in chunks of 37 for
+// the same reason, where 64 + 9 were padded to 128): 1143 us with 128 x 128 tiles and 64-spot chunks, 640
+// with these, 605-626 with three blocks to an SM (which small tiles allow and large ones do not: an
+// 8 x 8 register tile needs 128 registers).  A grid of 128 keeps its 128 x 128 tile: two of 64 x 128
+// would build every factor of the uncut axis twice.  Sums run in the same order whatever the tile.
+constexpr int kSizes[] = {4, 5, 6, 8};
+int tile_size(int n) {
+    const int nt = (n + kTile - 1) / kTile, need = ((n + nt - 1) / nt + 15) / 16;
+    for (int r : kSizes)
+        if (r >= need) return r;
+    return 8;
+}
 
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
@@ -101,18 +119,61 @@ __global__ void fwd_schedule_kernel(JobDev* jobs, FwdItem* items, int chunk) {
     }
 }
 
-__device__ __forceinline__ int xcol(int tx, int b) { return tx * 4 + (b & 3) + ((b >> 2) << 6); }
+// Tile of 16 RY rows x 16 RX columns, RY x RX voxels per thread: the first four of an axis are
+// consecutive (one 16-byte load), the others 16 apart past them (R < 8) or four more consecutive
+// ones (R = 8).
+template <int R>
+__device__ __forceinline__ int tcoord(int t, int b) {
+    if (b < 4) return 4 * t + b;
+    return R == 8 ? 64 + 4 * t + (b - 4) : 64 + t + 16 * (b - 4);
+}
+template <int R>
+__device__ __forceinline__ void tload(const float* row, int t, float (&v)[R]) {
+    const float4 a = *reinterpret_cast<const float4*>(row + 4 * t);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    if constexpr (R == 8) {
+        const float4 c = *reinterpret_cast<const float4*>(row + 64 + 4 * t);
+        v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
+    } else {
+#pragma unroll
+        for (int b = 4; b < R; ++b) v[b] = row[64 + t + 16 * (b - 4)];
+    }
+}
 
-__global__ void __launch_bounds__(NT, 2)
+// U[j, x] of a spot chunk: rows j = ty + 16 a, a < RJ (the chunk's rows, in groups of 16).
+template <int RJ, int RX>
+__device__ __forceinline__ void stage1(const float* WT, const float* GxT, int ni, int ty, int tx,
+                                       float (&uacc)[4][RX]) {
+#pragma unroll 2
+    for (int ii = 0; ii < ni; ++ii) {
+        float gb[RX];
+        tload<RX>(GxT + ii * 16 * RX, tx, gb);
+#pragma unroll
+        for (int a = 0; a < RJ; ++a) {
+            const float wa = WT[ii * SC + ty + 16 * a];
+#pragma unroll
+            for (int b = 0; b < RX; ++b) uacc[a][b] = fmaf(wa, gb[b], uacc[a][b]);
+        }
+    }
+}
+
+// Two blocks per SM for the largest tiles' registers, three for tiles up to 80 x 80: the barriers
+// and the weights' loads of one block run under the others' products.
+template <int RY, int RX>
+__global__ void __launch_bounds__(NT, RY * RX <= 25 ? 3 : 2)
 fwd_simt_kernel(const JobDev* __restrict__ jobs, const FwdItem* __restrict__ items, int total,
-                int* counter) {
+                int* counter, int sc) {
+    constexpr int TY = 16 * RY, TX = 16 * RX;
+    constexpr int PX = NT / TX, PY = NT / TY;        // spots generated at a time
     extern __shared__ float4 smem4[];
-    float* GxT = reinterpret_cast<float*>(smem4);   // [SC i][128 x]
-    float* GyT = GxT + SC * kTile;                   // [SC j][128 y]
-    float* U = GyT + SC * kTile;                     // [SC j][128 x]
-    float* WT = U + SC * kTile;                      // [SC i][SC j]
+    float* GxT = reinterpret_cast<float*>(smem4);   // [sc i][TX x]
+    float* GyT = GxT + sc * TX;                      // [sc j][TY y]
+    float* U = GyT + sc * TY;                        // [sc j][TX x]
+    float* WT = U + sc * TX;                         // [sc i][SC j]
     __shared__ int s_item;
+    __shared__ double s_xs[SC], s_ys[SC];
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    const int gx = tid % TX, gxr = tid / TX, gy = tid % TY, gyr = tid / TY;
 
     for (;;) {
         if (tid == 0) s_item = atomicAdd(counter, 1);
@@ -124,14 +185,15 @@ fwd_simt_kernel(const JobDev* __restrict__ jobs, const FwdItem* __restrict__ ite
         if (it.cost == 0) continue;
         const JobDev& J = jobs[it.job];
         const int nz = J.nz, nx = J.nx, ny = J.ny, nsx = J.nsx, nsy = J.nsy;
-        const int z = it.z, y0 = it.ty * kTile, x0 = it.tx * kTile;
+        const int z = it.z, y0 = it.ty * TY, x0 = it.tx * TX;
         const double cx = 0.5 * (double)(nsx - 1), cy = 0.5 * (double)(nsy - 1);
+        const double xv = J.ox + (double)(x0 + gx) * J.dx, yv = J.oy + (double)(y0 + gy) * J.dy;
 
-        float dacc[8][8];
+        float dacc[RY][RX];
 #pragma unroll
-        for (int a = 0; a < 8; ++a)
+        for (int a = 0; a < RY; ++a)
 #pragma unroll
-            for (int b = 0; b < 8; ++b) dacc[a][b] = 0.f;
+            for (int b = 0; b < RX; ++b) dacc[a][b] = 0.f;
 
         for (int l = it.lb; l < it.le; ++l) {
             const double c = J.idd[(size_t)l * nz + z];
@@ -141,72 +203,66 @@ fwd_simt_kernel(const JobDev* __restrict__ jobs, const FwdItem* __restrict__ ite
             const float nrm = (float)(c * kInv2Pi / (s * s));
             const float* wl = J.w + (size_t)l * nsy * nsx;
 
-            for (int j0 = 0; j0 < nsy; j0 += SC) {
-                const int nj = min(SC, nsy - j0);
-                float uacc[4][8];
+            for (int j0 = 0; j0 < nsy; j0 += sc) {
+                const int nj = min(sc, nsy - j0);
+                float uacc[4][RX];
 #pragma unroll
                 for (int a = 0; a < 4; ++a)
 #pragma unroll
-                    for (int b = 0; b < 8; ++b) uacc[a][b] = 0.f;
+                    for (int b = 0; b < RX; ++b) uacc[a][b] = 0.f;
 
-                for (int i0 = 0; i0 < nsx; i0 += SC) {
-                    const int ni = min(SC, nsx - i0);
+                for (int i0 = 0; i0 < nsx; i0 += sc) {
+                    const int ni = min(sc, nsx - i0);
                     __syncthreads();
-                    for (int e = tid; e < ni * kTile; e += NT) {
-                        const int ii = e >> 7, xx = e & (kTile - 1);
-                        const double d = (J.ox + (double)(x0 + xx) * J.dx) -
-                                         (J.sx0 + ((double)(i0 + ii) - cx) * J.dsx);
-                        GxT[e] = ex2_approx((float)(-(d * d) * a2));
-                    }
+                    // a thread forms the factors of one column (row) of the tile, every PX-th (PY-th)
+                    // spot: its voxel's position stays in a register
+                    if (tid < SC) s_xs[tid] = J.sx0 + ((double)(i0 + tid) - cx) * J.dsx;
+                    else if (tid < 2 * SC) s_ys[tid - SC] = J.sy0 + ((double)(j0 + tid - SC) - cy) * J.dsy;
+#pragma unroll 4
                     for (int e = tid; e < ni * SC; e += NT) {
                         const int ii = e / SC, jj = e % SC;
                         WT[e] = jj < nj ? nrm * wl[(size_t)(j0 + jj) * nsx + i0 + ii] : 0.f;
                     }
-                    if (i0 == 0) {
-                        for (int e = tid; e < nj * kTile; e += NT) {
-                            const int jj = e >> 7, yy = e & (kTile - 1);
-                            const double d = (J.oy + (double)(y0 + yy) * J.dy) -
-                                             (J.sy0 + ((double)(j0 + jj) - cy) * J.dsy);
-                            GyT[e] = ex2_approx((float)(-(d * d) * a2));
+                    __syncthreads();
+                    if (tid < PX * TX) {
+#pragma unroll 4
+                        for (int ii = gxr; ii < ni; ii += PX) {
+                            const double d = xv - s_xs[ii];
+                            GxT[ii * TX + gx] = ex2_approx((float)(-(d * d) * a2));
+                        }
+                    }
+                    if (i0 == 0 && tid < PY * TY) {
+#pragma unroll 4
+                        for (int jj = gyr; jj < nj; jj += PY) {
+                            const double d = yv - s_ys[jj];
+                            GyT[jj * TY + gy] = ex2_approx((float)(-(d * d) * a2));
                         }
                     }
                     __syncthreads();
                     // stage 1: U[j, x] += sum_i W'[j,i] Gx[x,i]
-                    for (int ii = 0; ii < ni; ++ii) {
-                        const float4 wv = *reinterpret_cast<const float4*>(&WT[ii * SC + ty * 4]);
-                        const float4 g0 = *reinterpret_cast<const float4*>(&GxT[ii * kTile + tx * 4]);
-                        const float4 g1 =
-                            *reinterpret_cast<const float4*>(&GxT[ii * kTile + 64 + tx * 4]);
-                        const float wa[4] = {wv.x, wv.y, wv.z, wv.w};
-                        const float gb[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-#pragma unroll
-                        for (int a = 0; a < 4; ++a)
-#pragma unroll
-                            for (int b = 0; b < 8; ++b) uacc[a][b] = fmaf(wa[a], gb[b], uacc[a][b]);
-                    }
+                    if (nj > 48) stage1<4, RX>(WT, GxT, ni, ty, tx, uacc);
+                    else if (nj > 32) stage1<3, RX>(WT, GxT, ni, ty, tx, uacc);
+                    else if (nj > 16) stage1<2, RX>(WT, GxT, ni, ty, tx, uacc);
+                    else stage1<1, RX>(WT, GxT, ni, ty, tx, uacc);
                 }
-                // U rows j = ty*4 + a
 #pragma unroll
                 for (int a = 0; a < 4; ++a) {
-                    float* row = U + (ty * 4 + a) * kTile;
-                    *reinterpret_cast<float4*>(&row[tx * 4]) =
-                        make_float4(uacc[a][0], uacc[a][1], uacc[a][2], uacc[a][3]);
-                    *reinterpret_cast<float4*>(&row[64 + tx * 4]) =
-                        make_float4(uacc[a][4], uacc[a][5], uacc[a][6], uacc[a][7]);
+                    if (ty + 16 * a >= nj) break;
+                    float* row = U + (ty + 16 * a) * TX;
+#pragma unroll
+                    for (int b = 0; b < RX; ++b) row[tcoord<RX>(tx, b)] = uacc[a][b];
                 }
                 __syncthreads();
                 // stage 2: D[y, x] += sum_j Gy[y,j] U[j,x]
+#pragma unroll 2
                 for (int jj = 0; jj < nj; ++jj) {
-                    const float4 q0 = *reinterpret_cast<const float4*>(&GyT[jj * kTile + ty * 8]);
-                    const float4 q1 = *reinterpret_cast<const float4*>(&GyT[jj * kTile + ty * 8 + 4]);
-                    const float4 u0 = *reinterpret_cast<const float4*>(&U[jj * kTile + tx * 4]);
-                    const float4 u1 = *reinterpret_cast<const float4*>(&U[jj * kTile + 64 + tx * 4]);
-                    const float ga[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-                    const float ub[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+                    float ga[RY], ub[RX];
+                    tload<RY>(GyT + jj * TY, ty, ga);
+                    tload<RX>(U + jj * TX, tx, ub);
 #pragma unroll
-                    for (int a = 0; a < 8; ++a)
+                    for (int a = 0; a < RY; ++a)
 #pragma unroll
-                        for (int b = 0; b < 8; ++b) dacc[a][b] = fmaf(ga[a], ub[b], dacc[a][b]);
+                        for (int b = 0; b < RX; ++b) dacc[a][b] = fmaf(ga[a], ub[b], dacc[a][b]);
                 }
             }
         }
@@ -214,12 +270,12 @@ fwd_simt_kernel(const JobDev* __restrict__ jobs, const FwdItem* __restrict__ ite
         const size_t n3 = (size_t)nz * ny * nx;
         float* out = J.partial + (size_t)it.chunk * n3 + (size_t)z * ny * nx;
 #pragma unroll
-        for (int a = 0; a < 8; ++a) {
-            const int y = y0 + ty * 8 + a;
+        for (int a = 0; a < RY; ++a) {
+            const int y = y0 + tcoord<RY>(ty, a);
             if (y >= ny) continue;
 #pragma unroll
-            for (int b = 0; b < 8; ++b) {
-                const int x = x0 + xcol(tx, b);
+            for (int b = 0; b < RX; ++b) {
+                const int x = x0 + tcoord<RX>(tx, b);
                 if (x < nx) out[(size_t)y * nx + x] = dacc[a][b];
             }
         }
@@ -257,6 +313,25 @@ __global__ void fwd_finalize_kernel(const JobDev* __restrict__ jobs, int with_lo
             __syncthreads();
         }
         if (threadIdx.x == 0) J.loss_part[blockIdx.x] = red[0];
+    }
+}
+
+using FwdKernel = void (*)(const JobDev*, const FwdItem*, int, int*, int);
+template <int RY>
+FwdKernel pick_rx(int rx) {
+    switch (rx) {
+        case 4: return fwd_simt_kernel<RY, 4>;
+        case 5: return fwd_simt_kernel<RY, 5>;
+        case 6: return fwd_simt_kernel<RY, 6>;
+        default: return fwd_simt_kernel<RY, 8>;
+    }
+}
+FwdKernel pick_kernel(int ry, int rx) {
+    switch (ry) {
+        case 4: return pick_rx<4>(rx);
+        case 5: return pick_rx<5>(rx);
+        case 6: return pick_rx<6>(rx);
+        default: return pick_rx<8>(rx);
     }
 }
 
@@ -309,15 +384,26 @@ int launch_forward(JobDev* jobs_dev, const JobDev* jobs_host, int n_jobs, FwdIte
         return launch_forward_tc(precision, jobs_dev, jobs_host, n_jobs, counter, err, chunk,
                                  with_loss, poison, s);
     }
-    int set = 0;
-    PBD_TRY(smem_optin((const void*)fwd_simt_kernel, (int)kFwdSmemBytes, 0, &set));
+    // one tile size per launch, the largest a job needs (the tile counts are the same for all)
+    int ry = kSizes[0], rx = kSizes[0], set = 0;
+    for (int j = 0; j < n_jobs; ++j) {
+        ry = std::max(ry, tile_size(jobs_host[j].ny));
+        rx = std::max(rx, tile_size(jobs_host[j].nx));
+    }
+    // spot chunks: the widest lattice in equal parts of at most 64 (73 spots as 37 + 36, not 64 + 9)
+    int ns = 1;
+    for (int j = 0; j < n_jobs; ++j) ns = std::max(ns, std::max(jobs_host[j].nsx, jobs_host[j].nsy));
+    const int parts = (ns + SC - 1) / SC, sc = ((ns + parts - 1) / parts + 3) / 4 * 4;
+    const FwdKernel kernel = pick_kernel(ry, rx);
+    PBD_TRY(smem_optin((const void*)kernel, (int)fwd_smem(ry, rx, SC), 0, &set));
     PBD_TRY(cuda_rc(cudaMemsetAsync(counter, 0, sizeof(int), s)));
     fwd_schedule_kernel<<<n_jobs, 256, kActStage, s>>>(jobs_dev, items, chunk);
     PBD_LAUNCH_CHECK();
     {
-        const int grid = max(1, min(total_items, 2 * num_sms()));
+        const int per_sm = ry * rx <= 25 && 3 * (fwd_smem(ry, rx, sc) + 2048u) <= 228u * 1024u ? 3 : 2;
+        const int grid = max(1, min(total_items, per_sm * num_sms()));
         prof_mark(kProfFwd, 0, s);
-        fwd_simt_kernel<<<grid, NT, kFwdSmemBytes, s>>>(jobs_dev, items, total_items, counter);
+        kernel<<<grid, NT, fwd_smem(ry, rx, sc), s>>>(jobs_dev, items, total_items, counter, sc);
         PBD_LAUNCH_CHECK();
         prof_mark(kProfFwd, 1, s);
     }
