@@ -77,7 +77,6 @@ constexpr int kMathWarps = 8;
 constexpr int kMath = 32 * kMathWarps;     // 256 math threads: warpgroups 0 and 1
 constexpr int kSchedWarp = kMathWarps;     // warpgroup 2: scheduler, two MMA warps, weight copies
 constexpr int kS1Warp = kMathWarps + 1;
-constexpr int kS2Warp = kMathWarps + 2;
 constexpr int kWWarp = kMathWarps + 3;
 constexpr int kThreads = kMath + 128;
 constexpr int kRing = 4;      // step slots (the largest two-tile shape leaves 1 KB of static shared memory)
@@ -600,7 +599,6 @@ __device__ __forceinline__ void store_b_sym(const Params& P, uint8_t* smem, uint
 template <bool kSplit>
 __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint32_t tb,
                                            const Step* ring, const Bars& B, unsigned (*s_gmax)[kMathWarps]) {
-    constexpr int NARR = kSplit ? 2 : 1;
     constexpr uint32_t kGt = 128u * 128u * 2u;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int sp = warp & 3, half = warp >> 2;

@@ -364,7 +364,7 @@ int fill_job(const pbd_field* f, JobDev* J) {
 // Jobs of one forward launch of the per-layer lateral maps: one single-layer job per layer,
 // depth dose 1 where the layer reaches the slice at all (`act`, (L, nz)), else 0.
 // Row stride (floats) of the per-layer lateral maps: the voxel count rounded up to 64 floats,
-// so every row starts on a 256-byte boundary for the combine's bulk copies.
+// so every row starts on a 256-byte boundary.
 static size_t wed_lateral_stride(const pbd_field* f) {
     return align_up((size_t)f->nz * f->ny * f->nx, 64);
 }
@@ -384,8 +384,15 @@ static void wed_jobs(const pbd_field* f, int l0, int n, const float* w, const do
     }
 }
 
+// The lateral maps' forward: TF32x3 callers get the split-FP16 kernel, which has the same 22-bit
+// operands, half the tensor work and a smaller error (128^3, 40 layers: 85 us against 262, dose 1.3e-7
+// against 2.7e-7 of 64 bits).  The single-product and BF16 precisions keep their own kernel.
+static int wed_map_precision(int precision) {
+    return precision == PBD_PREC_TF32X3 ? PBD_PREC_FP16X3 : precision;
+}
+
 struct WedCarve {
-    int* status;         // status header: forward, combine error words
+    int* status;         // status header: the forward's error word
     double* act;
     float* lateral;      // (L, wed_lateral_stride) per-layer lateral maps
     void* curves;
@@ -405,7 +412,7 @@ static int carve_wed(const pbd_field* f, const pbd_lut_spec* spec, int precision
         PBD_TRY(pbd_forward_batch_workspace(jobs, nb, precision, &bb));
     } else {
         Ws fw;
-        PBD_TRY(carve_ws(f, true, false, false, precision, nullptr, fw, &bb));
+        PBD_TRY(carve_ws(f, true, false, false, wed_map_precision(precision), nullptr, fw, &bb));
     }
     PBD_TRY(lut_curve_workspace(spec, L, &cb));
     Carve c(base);
@@ -959,6 +966,7 @@ int pbd_build_wed_curves(const pbd_lut_spec* spec, int n_layers, const double* e
 static int forward_layer_maps(const pbd_field* f, const float* w, const double* act,
                               const double* sigma, float* lateral, size_t lstride, int precision,
                               void* base, size_t bytes, cudaStream_t s, int* err) {
+    precision = wed_map_precision(precision);
     size_t need = 0;
     Ws ws;
     PBD_TRY(carve_ws(f, true, false, false, precision, nullptr, ws, &need));
@@ -977,9 +985,9 @@ static int forward_layer_maps(const pbd_field* f, const float* w, const double* 
     install_jobs_kernel<<<1, 32, 0, s>>>(p, ws.jobs, nullptr);
     PBD_LAUNCH_CHECK();
     count_launch(1);
-    // no poison pass here: the combine's poison pass reads this error word too
+    // no poison pass here: the combine reads this error word
     return launch_forward(ws.jobs, &J, 1, ws.fitems, ws.f_items, ws.counters, ws.n_fcount, err,
-                          ws.f_chunk, 0, precision, 0, nullptr, 0, s);
+                          ws.f_chunk, 0, precision, 0, ws.pack, ws.pack_bytes, s);
 }
 
 // Activity table, the per-layer lateral maps, then the combine.
@@ -1008,7 +1016,7 @@ static int forward_wed_body(const pbd_field* f, const pbd_lut_spec* spec, const 
         }
     }
     return lut_wed_combine(spec, f->n_layers, wc.lateral, lstride, wed, (size_t)f->nz * nslice,
-                           dose, wc.status + kStatCmb, fwd_err, curves, curves_bytes, s);
+                           dose, fwd_err, curves, curves_bytes, s);
 }
 
 static int wed_setup(const pbd_field* f, const pbd_lut_spec* spec, int precision, void* workspace,

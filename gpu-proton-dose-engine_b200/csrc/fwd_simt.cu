@@ -371,7 +371,7 @@ int launch_forward(JobDev* jobs_dev, const JobDev* jobs_host, int n_jobs, FwdIte
                    int total_items, int* counter, size_t n_counter_ints, int* err, int chunk,
                    int with_loss, int precision, int poison, void* pack, size_t pack_bytes,
                    cudaStream_t s, const JobPair* inst, JobDev* inst_dst, int* inst_status) {
-    const bool tc16 = precision == PBD_PREC_FP16X3 && jobs_host[0].layer_stride == 0;
+    const bool tc16 = precision == PBD_PREC_FP16X3;
     if (inst && !tc16) return PBD_ERR_UNSUPPORTED;   // only the split-FP16 pack installs views
     if (precision != PBD_PREC_FP32) {
         // the split-FP16 path clears its unit counter in its pack kernel (no memset node between

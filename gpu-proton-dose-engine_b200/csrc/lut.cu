@@ -591,186 +591,100 @@ lut_eval_kernel(pbd_lut_spec spec, LutDims dm, const LayerScal* __restrict__ sca
 // Heterogeneous media: dose = sum_l IDD_l(WED) * lateral_l per voxel, IDD_l the layer's
 // smoothed depth curve evaluated at the voxel's water-equivalent depth with the same
 // interpolation as the tables (lut_output_kernel).  Accumulated in FP64, in layer order.
-constexpr int kWedLayers = 256;   // layers whose curve scalars are staged in shared memory
-
-// The combine streams each layer's lateral values of a 1024-voxel tile into a ring of
-// shared-memory stages with 1-D bulk copies (cp.async.bulk, completion on an mbarrier), so the
-// bytes in flight do not depend on the registers the FP64 interpolation needs.  Layers that
-// no voxel of the tile reaches (tile's smallest WED above zmax, or largest below 0) are
-// neither copied nor evaluated.  Waits are bounded (2 s); a block whose wait runs out sets
-// the error word, waits (bounded) for its own copies in flight and leaves, and the poison pass
-// turns the dose into NaN.
+//
+// A warp owns 128 consecutive voxels (4 per lane, lanes adjacent) and walks the layers that reach any
+// of them, the next layer's lateral values loaded while this one's curve points are gathered; layers
+// that reach none (smallest WED above zmax) are neither read nor evaluated.  A voxel counts only where
+// its WED lies inside the curve (or is NaN): outside [0, zmax] nothing is added, and a (layer, slice)
+// the activity table marked inactive has every WED above zmax, so the unwritten part of a lateral map
+// is loaded at most, never used.
+//
+// Bound by the gathers of curve points through L1 (neighbouring columns differ by the CT's noise) and
+// instruction issue.  The interval is the rounded estimate alone, without the correction to np.interp's
+// exact choice: the interpolation is continuous, so an estimate one interval off within rounding of a
+// knot gives the same value to FP64 rounding.  128^3, 40 layers: 195 us with the corrected interval and
+// the lateral values in a ring of bulk copies with a block barrier per layer (90 instructions per voxel
+// and layer), 98 us now (L1 gathers about 60).
 constexpr int kCmbThreads = 256;
-constexpr int kCmbPer = 4;                              // voxels per thread
-constexpr int kCmbTile = kCmbThreads * kCmbPer;         // voxels per tile (4 KB of one layer)
-constexpr int kCmbStages = 6;
+constexpr int kCmbPer = 4;                              // voxels per lane
+constexpr int kCmbTile = kCmbThreads * kCmbPer;         // voxels per block
+constexpr int kCmbLayers = 128;                         // layers whose scalars are staged at a time
 
-__device__ __forceinline__ void bulk_load_s(void* dst, const void* src, uint32_t bytes,
-                                            uint64_t* bar) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(bar)),
-                 "r"(bytes)
-                 : "memory");
-    asm volatile(
-        "cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            tc::smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(tc::smem_u32(bar))
-        : "memory");
-}
-
-// 48 registers, no spills: 5 blocks per SM (64 registers without the bound: 4)
-__global__ void __launch_bounds__(kCmbThreads, 5) wed_combine_kernel(
-    LutDims dm, const LayerScal* scal, const double2* pts, const float* lateral, size_t lstride,
-    const double* wed, size_t nvox, int n_layers, float* dose, int* err) {
-    __shared__ __align__(128) float lat[kCmbStages][kCmbTile];
-    __shared__ __align__(8) uint64_t full[kCmbStages];
-    __shared__ double zmax[kWedLayers], stp[kWedLayers], istp[kWedLayers];
-    __shared__ double rmin[kCmbThreads / 32], rmax[kCmbThreads / 32];
-    __shared__ int rnan[kCmbThreads / 32];
-    __shared__ int abort_s;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int l = tid; l < n_layers && l < kWedLayers; l += kCmbThreads) {
-        zmax[l] = scal[l].zmax;
-        stp[l] = (scal[l].zmax - 0.0) / (double)(dm.n_idd - 1);
-        istp[l] = 1.0 / stp[l];
-    }
-    if (tid == 0) {
-        for (int q = 0; q < kCmbStages; ++q) tc::mbar_init(&full[q], 1);
-        tc::fence_mbar_init();
-        abort_s = 0;
-    }
-    __syncthreads();
-    const int n = dm.n_idd;
+__global__ void __launch_bounds__(kCmbThreads, 4) wed_combine_kernel(
+    int n, const LayerScal* __restrict__ scal, const double2* __restrict__ pts,
+    const float* __restrict__ lateral, size_t lstride, const double* __restrict__ wed, size_t nvox,
+    int n_layers, float* __restrict__ dose, const int* __restrict__ fwd_err) {
+    __shared__ double s_zmax[kCmbLayers], s_step[kCmbLayers], s_inv[kCmbLayers];
+    const int lane = threadIdx.x & 31;
+    const size_t v0 = (size_t)blockIdx.x * kCmbTile + (threadIdx.x >> 5) * (32 * kCmbPer) + lane;
     const double inf = __longlong_as_double(0x7FF0000000000000ll);
-    const size_t n_tiles = (nvox + kCmbTile - 1) / kCmbTile;
-    uint32_t it = 0;       // copies consumed: stage it % kCmbStages, parity (it / kCmbStages) & 1
-    uint32_t issued = 0;   // copies issued (thread 0)
-    int next_l = 0;        // next layer thread 0 considers (thread 0)
-    for (size_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-        const size_t v0 = t * kCmbTile;
-        const int cnt = (int)((nvox - v0) < (size_t)kCmbTile ? (nvox - v0) : (size_t)kCmbTile);
-        double d[kCmbPer], acc[kCmbPer];
-        double mn = inf, mx = -inf;
-        int has_nan = 0;
+    constexpr double kMagic = 6755399441055744.0;       // 1.5 2^52: the sum's low word is the integer
+    double d[kCmbPer], acc[kCmbPer], mn = inf;
+    size_t at[kCmbPer];
 #pragma unroll
-        for (int j = 0; j < kCmbPer; ++j) {
-            const int i = tid + j * kCmbThreads;
-            acc[j] = 0.0;
-            d[j] = 0.0;
-            if (i < cnt) {
-                d[j] = __ldcs(wed + v0 + i);
-                if (d[j] != d[j]) {
-                    has_nan = 1;
-                } else {
-                    mn = fmin(mn, d[j]);
-                    mx = fmax(mx, d[j]);
-                }
-            }
-        }
+    for (int j = 0; j < kCmbPer; ++j) {
+        const size_t v = v0 + 32 * j;
+        at[j] = v < nvox ? v : nvox - 1;
+        d[j] = __ldcs(wed + at[j]);
+        if (v >= nvox || d[j] < 0.0) d[j] = inf;        // inside no curve
+        mn = d[j] != d[j] ? -inf : fmin(mn, d[j]);      // a NaN takes every layer
+        acc[j] = 0.0;
+    }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            has_nan |= __shfl_xor_sync(0xffffffffu, has_nan, o);
-        }
-        if (lane == 0) {
-            rmin[warp] = mn;
-            rmax[warp] = mx;
-            rnan[warp] = has_nan;
+    for (int o = 16; o > 0; o >>= 1) mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    for (int b = 0; b < n_layers; b += kCmbLayers) {
+        const int nb = min(kCmbLayers, n_layers - b);
+        __syncthreads();
+        for (int l = threadIdx.x; l < nb; l += kCmbThreads) {
+            s_zmax[l] = scal[b + l].zmax;
+            s_step[l] = scal[b + l].step;
+            s_inv[l] = scal[b + l].inv;
         }
         __syncthreads();
-        double tmin = inf, tmax = -inf;
-        bool tnan = false;
-#pragma unroll
-        for (int q = 0; q < kCmbThreads / 32; ++q) {
-            tmin = fmin(tmin, rmin[q]);
-            tmax = fmax(tmax, rmax[q]);
-            tnan = tnan || rnan[q] != 0;
-        }
-        // the same answer in every thread: layer l is copied and evaluated for this tile
-        auto active = [&](int l) -> bool {
-            const double zm = l < kWedLayers ? zmax[l] : scal[l].zmax;
-            return tnan || (tmin <= zm && tmax >= 0.0);
+        auto next = [&](int l) {
+            while (l < nb && !(mn <= s_zmax[l])) ++l;
+            return l;
         };
-        const uint32_t bytes = (uint32_t)((cnt + 3) / 4) * 16u;
-        auto refill = [&]() {
-            while (issued - it < (uint32_t)kCmbStages && next_l < n_layers) {
-                if (active(next_l)) {
-                    const uint32_t q = issued % kCmbStages;
-                    bulk_load_s(lat[q], lateral + (size_t)next_l * lstride + v0, bytes, &full[q]);
-                    ++issued;
-                }
-                ++next_l;
-            }
+        float lat[kCmbPer];
+        auto fetch = [&](int l, float* x) {
+            const float* p = lateral + (size_t)(b + l) * lstride;
+#pragma unroll
+            for (int j = 0; j < kCmbPer; ++j) x[j] = __ldcs(p + at[j]);
         };
-        if (tid == 0) {
-            next_l = 0;
-            refill();
-        }
-        for (int l = 0; l < n_layers; ++l) {
-            if (!active(l)) continue;
-            const uint32_t q = it % kCmbStages;
-            if (!tcc::wait_bar(&full[q], (it / kCmbStages) & 1u)) {
-                abort_s = 1;
-                atomicExch(err, 1);
-            } else {
-                const double zm = l < kWedLayers ? zmax[l] : scal[l].zmax;
-                const double st = l < kWedLayers ? stp[l] : (zm - 0.0) / (double)(n - 1);
-                const double is = l < kWedLayers ? istp[l] : 1.0 / st;
-                const double2* lp = pts + (size_t)l * n;
-                // A voxel counts only where its WED lies inside the curve (or is NaN): outside
-                // [0, zmax] the curve's fill values are 0 and nothing is added, and a (layer,
-                // slice) the activity table marked inactive has every WED above zmax, so the
-                // unwritten part of a lateral map is copied at most, never used.
-                int lo[kCmbPer];
-                double x0[kCmbPer];
+        int l = next(0);
+        if (l < nb) fetch(l, lat);
+        while (l < nb) {
+            const int ln = next(l + 1);
+            float ahead[kCmbPer];
 #pragma unroll
-                for (int j = 0; j < kCmbPer; ++j) {
-                    lo[j] = 0;
-                    x0[j] = 0.0;
-                    if (tid + j * kCmbThreads < cnt && !(d[j] < 0.0 || d[j] > zm))
-                        locate_curve(d[j], zm, n, st, is, lo[j], x0[j]);
-                }
+            for (int j = 0; j < kCmbPer; ++j) ahead[j] = 0.f;
+            if (ln < nb) fetch(ln, ahead);
+            const double zm = s_zmax[l], st = s_step[l], inv = s_inv[l];
+            const double2* lp = pts + (size_t)(b + l) * n;
+            double2 pt[kCmbPer];
+            double x[kCmbPer];
 #pragma unroll
-                for (int j = 0; j < kCmbPer; ++j) {
-                    const int i = tid + j * kCmbThreads;
-                    if (i >= cnt || d[j] < 0.0 || d[j] > zm) continue;
-                    const double2 pt = __ldg(lp + lo[j]);
-                    // np.interp's value: fp[lo] on a grid point, else slope * (x - x0) + fp[lo]
-                    // with the slope np.interp rounds; the sum in layer order
-                    const double idd = x0[j] == d[j] ? pt.x : pt.y * (d[j] - x0[j]) + pt.x;
-                    if (idd == 0.0) continue;
-                    acc[j] += idd * (double)lat[q][i];
-                }
+            for (int j = 0; j < kCmbPer; ++j) {
+                const double t = fma(d[j], inv, -0.5) + kMagic;
+                const unsigned lo = min((unsigned)__double2loint(t), (unsigned)(n - 1));
+                x[j] = fma(kMagic - t, st, d[j]);       // from the interval's left point
+                pt[j] = __ldg(lp + lo);
             }
-            __syncthreads();   // stage q is free again; abort_s is visible to every thread
-            ++it;
-            if (abort_s) break;
-            if (tid == 0) refill();
-        }
-        if (abort_s) {
-            // the copies still in flight (the one whose wait ran out included) land before
-            // the block's shared memory is released
-            if (tid == 0)
-                for (uint32_t c = it - 1; c != issued; ++c)
-                    (void)tcc::wait_bar(&full[c % kCmbStages], (c / kCmbStages) & 1u);
-            return;
-        }
 #pragma unroll
-        for (int j = 0; j < kCmbPer; ++j) {
-            const int i = tid + j * kCmbThreads;
-            if (i < cnt) __stcs(dose + v0 + i, (float)acc[j]);
+            for (int j = 0; j < kCmbPer; ++j) {
+                const double idd = fma(pt[j].y, x[j], pt[j].x);
+                if (!(d[j] > zm) && idd != 0.0) acc[j] = fma(idd, (double)lat[j], acc[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < kCmbPer; ++j) lat[j] = ahead[j];
+            l = ln;
         }
-        __syncthreads();   // the next tile's reduction reuses rmin / rmax / rnan
     }
-}
-
-// After a combine (or the lateral maps' forward, err2) whose wait ran out: the whole dose is
-// invalid, NaN.
-__global__ void wed_poison_kernel(float* dose, size_t nvox, const int* err, const int* err2) {
-    if (*err == 0 && (err2 == nullptr || *err2 == 0)) return;
-    for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nvox;
-         v += (size_t)gridDim.x * blockDim.x)
-        dose[v] = __int_as_float(0x7fc00000);
+    // a wait of the lateral maps' forward ran out: the whole dose is invalid
+    const bool bad = fwd_err && *fwd_err;
+#pragma unroll
+    for (int j = 0; j < kCmbPer; ++j)
+        if (v0 + 32 * j < nvox) __stcs(dose + v0 + 32 * j, bad ? __int_as_float(0x7fc00000) : (float)acc[j]);
 }
 
 // Depth dose of a layer's curve {value, slope} at depth d (np.interp's interval and value, 0
@@ -951,31 +865,59 @@ __global__ void __launch_bounds__(kActThreads) wed_activity_kernel(const LayerSc
 // Water-equivalent depth at the voxel centres z_k = oz + k dz along +z (the beam axis):
 // the sum of rho * path length from depth 0 (physics.py:421-423 per voxel path), voxel i
 // filling [z_i - dz/2, z_i + dz/2] with rho_i, water above the first voxel, path lengths
-// clipped at depth 0.  One thread per (y, x) column, FP64, in depth order.
-constexpr int kRayThreads = 64;   // 64-thread blocks: a 128 x 128 field still fills every SM
-constexpr int kRayBatch = 16;     // depths whose rho one thread loads before the running sum
+// clipped at depth 0.  FP64.
+//
+// A block holds 32 columns and 16 runs of 8 depths (one per warp): each thread sums its run, the sums
+// of the runs above are added through shared memory, 128 depths at a time.  Bound by the latency of the
+// loads: one thread per column had 16 of them in flight in 4 warps per SM (128^3: 31 us), now 8 in
+// 32 warps (12 us).
+constexpr int kRayCols = 32, kRayRuns = 16, kRayLen = 8;
 
-__global__ void __launch_bounds__(kRayThreads) wed_raytrace_kernel(int nz, size_t ncol, double oz,
-                                                                   double dz, const float* rho,
-                                                                   double* wed) {
-    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncol;
-         c += (size_t)gridDim.x * blockDim.x) {
-        const double top0 = oz - 0.5 * dz;
-        double acc = top0 > 0.0 ? top0 : 0.0;          // water above the first voxel
-        for (int k0 = 0; k0 < nz; k0 += kRayBatch) {
-            float r[kRayBatch];
+__global__ void __launch_bounds__(kRayCols * kRayRuns, 2) wed_raytrace_kernel(int nz, size_t ncol, double oz,
+                                                                           double dz,
+                                                                           const float* __restrict__ rho,
+                                                                           double* __restrict__ wed) {
+    __shared__ double sums[2][kRayRuns][kRayCols];
+    const int lane = threadIdx.x & 31, run = threadIdx.x >> 5;
+    auto depths = [&](int k, double& lo, double& mid, double& hi) {
+        const double zc = oz + (double)k * dz;
+        lo = fmax(zc - 0.5 * dz, 0.0);
+        mid = fmax(zc, 0.0);
+        hi = fmax(zc + 0.5 * dz, 0.0);
+    };
+    int buf = 0;
+    for (size_t c0 = (size_t)blockIdx.x * kRayCols; c0 < ncol; c0 += (size_t)gridDim.x * kRayCols) {
+        const size_t c = c0 + lane;
+        const bool in = c < ncol;
+        double above = fmax(oz - 0.5 * dz, 0.0);         // water above the first voxel
+        for (int k0 = 0; k0 < nz; k0 += kRayRuns * kRayLen) {
+            const int kr = k0 + run * kRayLen;
+            float r[kRayLen];
 #pragma unroll
-            for (int q = 0; q < kRayBatch; ++q)
-                r[q] = k0 + q < nz ? __ldcs(rho + (size_t)(k0 + q) * ncol + c) : 0.0f;
+            for (int q = 0; q < kRayLen; ++q)
+                r[q] = in && kr + q < nz ? __ldcs(rho + (size_t)(kr + q) * ncol + c) : 0.f;
+            double sum = 0.0;
 #pragma unroll
-            for (int q = 0; q < kRayBatch; ++q) {
-                const int k = k0 + q;
-                if (k >= nz) break;
-                const double zc = oz + (double)k * dz;
-                const double lo = fmax(zc - 0.5 * dz, 0.0), mid = fmax(zc, 0.0);
-                const double hi = fmax(zc + 0.5 * dz, 0.0);
+            for (int q = 0; q < kRayLen; ++q) {
+                double lo, mid, hi;
+                depths(kr + q, lo, mid, hi);
+                sum += (double)r[q] * (hi - lo);
+            }
+            sums[buf][run][lane] = sum;
+            __syncthreads();
+            double acc = above;
+#pragma unroll 4
+            for (int w = 0; w < kRayRuns; ++w) {
+                if (w == run) acc = above;
+                above += sums[buf][w][lane];
+            }
+            buf ^= 1;                                    // the next pass's sums: no barrier here
+#pragma unroll
+            for (int q = 0; q < kRayLen; ++q) {
+                double lo, mid, hi;
+                depths(kr + q, lo, mid, hi);
                 const double rr = (double)r[q];
-                __stcs(wed + (size_t)k * ncol + c, acc + rr * (mid - lo));
+                if (in && kr + q < nz) __stcs(wed + (size_t)(kr + q) * ncol + c, acc + rr * (mid - lo));
                 acc += rr * (hi - lo);
             }
         }
@@ -1230,36 +1172,21 @@ int lut_wed_activity(const pbd_lut_spec* s, int n_layers, const void* curves, si
 }
 
 int lut_wed_combine(const pbd_lut_spec* s, int n_layers, const float* lateral, size_t lstride,
-                    const double* wed, size_t nvox, float* dose, int* err, const int* err2,
+                    const double* wed, size_t nvox, float* dose, const int* fwd_err,
                     const void* curves, size_t curves_bytes, cudaStream_t st) {
     PBD_TRY(validate_spec(s, n_layers));
-    if (!lateral || !wed || !dose || !err) return PBD_ERR_NULL_ARG;
-    // 1-D bulk copies: 16-byte aligned rows, the tile's copy rounded up to 16 bytes inside
-    // the row
-    if ((reinterpret_cast<size_t>(lateral) & 15) || (lstride & 3) || lstride < ((nvox + 3) & ~(size_t)3))
-        return PBD_ERR_BAD_VALUE;
+    if (!lateral || !wed || !dose) return PBD_ERR_NULL_ARG;
+    if (lstride < nvox) return PBD_ERR_BAD_VALUE;
     LutDims dm;
     LutWs w;
     double2* pts = nullptr;
     PBD_TRY(wed_dims(s, n_layers, curves, curves_bytes, dm, w, pts));
-    static int per_sm = 0;
-    if (per_sm == 0) {
-        int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, wed_combine_kernel, kCmbThreads, 0) !=
-                cudaSuccess || b < 1)
-            b = 1;
-        per_sm = b;
-    }
-    const size_t n_tiles = (nvox + kCmbTile - 1) / kCmbTile;
-    const int blocks = (int)std::min<size_t>(n_tiles, (size_t)num_sms() * per_sm);
-    wed_combine_kernel<<<std::max(blocks, 1), kCmbThreads, 0, st>>>(dm, w.scal, pts, lateral,
-                                                                    lstride, wed, nvox, n_layers,
-                                                                    dose, err);
+    const size_t blocks = (nvox + kCmbTile - 1) / kCmbTile;
+    if (blocks > 0x7fffffffu) return PBD_ERR_UNSUPPORTED;
+    wed_combine_kernel<<<(unsigned)blocks, kCmbThreads, 0, st>>>(dm.n_idd, w.scal, pts, lateral, lstride, wed,
+                                                                 nvox, n_layers, dose, fwd_err);
     PBD_LAUNCH_CHECK();
-    const int pb = (int)std::min<size_t>((nvox + 255) / 256, (size_t)num_sms() * 4);
-    wed_poison_kernel<<<std::max(pb, 1), 256, 0, st>>>(dose, nvox, err, err2);
-    PBD_LAUNCH_CHECK();
-    count_launch(2);
+    count_launch(1);
     return PBD_OK;
 }
 
@@ -1300,9 +1227,8 @@ int lut_wed_raytrace(int nz, int ny, int nx, double oz, double dz, const float* 
     if (nz <= 0 || ny <= 0 || nx <= 0) return PBD_ERR_BAD_DIM;
     if (!isfinite(oz) || !(dz > 0.0) || !isfinite(dz)) return PBD_ERR_BAD_VALUE;
     const size_t ncol = (size_t)ny * nx;
-    const int blocks = (int)std::min<size_t>((ncol + kRayThreads - 1) / kRayThreads,
-                                             (size_t)num_sms() * 32);
-    wed_raytrace_kernel<<<std::max(blocks, 1), kRayThreads, 0, st>>>(nz, ncol, oz, dz, rho, wed);
+    const int blocks = (int)std::min<size_t>((ncol + kRayCols - 1) / kRayCols, (size_t)num_sms() * 32);
+    wed_raytrace_kernel<<<blocks, kRayCols * kRayRuns, 0, st>>>(nz, ncol, oz, dz, rho, wed);
     PBD_LAUNCH_CHECK();
     count_launch(1);
     return PBD_OK;

@@ -149,11 +149,10 @@ int loss_partials(const pbd_field* f, int precision);
 
 // Status header: the first sub-array of every workspace whose kernels run bounded waits
 // (kStatusInts ints at the workspace's first 256-byte boundary).  Word kStatFwd is the
-// forward's error word, kStatAdj the adjoint's, kStatCmb the heterogeneous combine's; the
-// call's first kernel (or memset) clears the header, a wait that runs out sets its word, and
-// pbd_workspace_status() reads them back.
+// forward's error word, kStatAdj the adjoint's; the call's first kernel (or memset) clears the
+// header, a wait that runs out sets its word, and pbd_workspace_status() reads them back.
 constexpr int kStatusInts = 16;
-enum StatusWord { kStatFwd = 0, kStatAdj = 1, kStatCmb = 2 };
+enum StatusWord { kStatFwd = 0, kStatAdj = 1 };
 
 // Dynamic shared memory opt-in of kernel `fn` on the CURRENT device, done once per (device,
 // kernel) and cached: bytes >= 0 sets that size; bytes < 0 sets the device's opt-in maximum
@@ -253,10 +252,8 @@ int lut_csda(const double* e, double* r, int n, int inverse, cudaStream_t st);
 // Heterogeneous media (lut.cu): size of the depth-curve blob; curves builds the per-layer
 // smoothed depth curves and their interval slopes into it; activity fills the (layer, slice)
 // table act (L, nz) from a WED map; combine forms dose = sum_l IDD_l(WED) * lateral_l with
-// layer l's lateral map at lateral + l * lstride (16-byte aligned, lstride a multiple of 4
-// floats, >= nvox rounded up to 4), its error word err (set when a bounded wait ran out) and
-// optionally the lateral maps' forward error word err2 (either one makes the dose NaN); the
-// WED ray trace along +z.
+// layer l's lateral map at lateral + l * lstride (>= nvox) and optionally the lateral maps'
+// forward error word (when set, the dose is NaN); the WED ray trace along +z.
 int lut_curve_workspace(const pbd_lut_spec* s, int n_layers, size_t* bytes);
 int lut_wed_curves(const pbd_lut_spec* s, int n_layers, const double* energies,
                    const double* shift, void* curves, size_t curves_bytes, cudaStream_t st);
@@ -266,7 +263,7 @@ int lut_wed_activity(const pbd_lut_spec* s, int n_layers, const void* curves, si
                      const double* wed, int nz, size_t nslice, double* act, cudaStream_t st,
                      const void* curves2 = nullptr, size_t curves2_bytes = 0);
 int lut_wed_combine(const pbd_lut_spec* s, int n_layers, const float* lateral, size_t lstride,
-                    const double* wed, size_t nvox, float* dose, int* err, const int* err2,
+                    const double* wed, size_t nvox, float* dose, const int* fwd_err,
                     const void* curves, size_t curves_bytes, cudaStream_t st);
 // maps (L, lstride): dL/dD times each layer's depth dose at the WED (the heterogeneous adjoint's
 // per-layer input), written on the slices that act (L, nz) marks.  With curves_p / curves_m (the

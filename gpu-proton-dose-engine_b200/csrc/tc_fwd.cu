@@ -1006,12 +1006,11 @@ int launch_forward_tc(int precision, JobDev* jobs_dev, const JobDev* jobs_host, 
     for (int j = 1; j < n_jobs; ++j)
         if ((jobs_host[j].layer_stride != 0) != maps) return PBD_ERR_UNSUPPORTED;
     if (maps && with_loss) return PBD_ERR_UNSUPPORTED;
-    // the split-FP16 kernel has no per-layer-maps mode: its accuracy class is TF32x3's
-    if (precision == PBD_PREC_FP16X3) precision = PBD_PREC_TF32X3;
     int rc = PBD_ERR_BAD_VALUE;
     switch (precision) {
         case PBD_PREC_TF32X3:
-            rc = maps ? launch_mode<PBD_PREC_TF32X3, true>(P, s) : launch_mode<PBD_PREC_TF32X3, false>(P, s);
+            // TF32x3 callers' maps come from the split-FP16 kernel
+            rc = maps ? PBD_ERR_UNSUPPORTED : launch_mode<PBD_PREC_TF32X3, false>(P, s);
             break;
         case PBD_PREC_TF32:
             rc = maps ? launch_mode<PBD_PREC_TF32, true>(P, s) : launch_mode<PBD_PREC_TF32, false>(P, s);

@@ -45,6 +45,13 @@
 // that the math warps add in FP32 registers (the tensor core truncates when it accumulates),
 // the cross products (~2^-11 of them) stay in one accumulator per unit.
 //
+// Per-layer maps (jobs with layer_stride > 0: the lateral maps of a dose in a medium, FP16x3 and
+// TF32x3 callers): every step is its own output, with its own scale exponent.  One MMA warp issues all
+// of stage 2 into the step's accumulator, cross products first, so that the unit's cross accumulator
+// and its drain fall away; a lane stores 32 bytes at a time.  128^3, 41 x 41 x 40: 85 us, of which the
+// 200 MB written take 31; the TF32x3 kernel's maps took 262 (twice the MMAs at half the rate, straight
+// line phases, 16-byte stores) and were twice as far from 64 bits (dose 2.7e-7 against 1.3e-7).
+//
 // Output (per math warp: 32 rows x 64 columns of the tile): plain stores of the unit's partial
 // slice (or, where every unit holds all layers of its slice, of the dose itself); a finalize
 // pass then sums each voxel's partials in chunk order -- deterministic -- and, with the loss,
@@ -68,9 +75,7 @@ using namespace tcc;
 constexpr int kMathWarps = kTcFwdWarps;
 constexpr int kMath = 32 * kMathWarps;     // 256 math threads: warpgroups 0 and 1
 constexpr int kSchedWarp = kMathWarps;     // warpgroup 2: scheduler / producer, then 3 MMA warps
-constexpr int kS1Warp = kMathWarps + 1;
-constexpr int kS2Warp = kMathWarps + 2;
-constexpr int kS3Warp = kMathWarps + 3;
+constexpr int kS3Warp = kMathWarps + 3;    // stage 2's cross products
 constexpr int kThreads = kMath + 128;
 constexpr int kMathRegs = 208, kCtrlRegs = 80;
 constexpr int kLaunchRegsNeeded = (kMath * kMathRegs + 128 * kCtrlRegs + kThreads - 1) / kThreads;
@@ -240,6 +245,7 @@ __global__ void __launch_bounds__(256) pack_w16_kernel(const JobDev* __restrict_
 // ------------------------------------------------------------------------------------------
 // Scheduler / producer warp.
 // ------------------------------------------------------------------------------------------
+template <bool MAPS>
 __device__ __forceinline__ void scheduler_warp(const Params& P, uint8_t* smem, Step* ring,
                                                uint64_t* full, uint64_t* empty, uint64_t* wfull,
                                                uint64_t* wempty) {
@@ -325,11 +331,11 @@ __device__ __forceinline__ void scheduler_warp(const Params& P, uint8_t* smem, S
             const int nch = (tot + P.chunk - 1) / P.chunk;
             // the finalize pass sums nch partial slices of slice z (every unit of the slice
             // writes the same count)
-            if (!J.direct && c == 0 && tile == 0 && lane == 0) J.nchunks[z] = nch;
+            if (!MAPS && !J.direct && c == 0 && tile == 0 && lane == 0) J.nchunks[z] = nch;
             if (tot == 0) {
                 // a slice no layer reaches: zeros written here when the output is the dose
                 // itself, else by the finalize pass (zero partial slices)
-                if (c == 0 && J.direct) {
+                if (!MAPS && c == 0 && J.direct) {
                     Step st{};
                     st.job = job; st.z = z; st.tile = tile;
                     st.nch = 1; st.flags = kFirst | kLast | kZero;
@@ -342,27 +348,26 @@ __device__ __forceinline__ void scheduler_warp(const Params& P, uint8_t* smem, S
             // the unit's scale exponent: the smallest over its layers of
             // 14 - ceil(log2(bound on |s U|)), so that every s U of the unit fits FP16
             int ks = 127;
-            {
+            auto scale = [&](double iv, double s, float wm) {
+                const double bnd = fabs(iv) * kInv2Pi / (s * s) * (double)wm *
+                                   (1.0 + 2.5066282746310002 * s / J.dsx);
+                int q = 0;
+                if (!(bnd > 0.0 && bnd < 1e300)) return 127;
+                (void)frexp(bnd, &q);          // bnd < 2^q
+                return 14 - q;
+            };
+            auto clamp = [](int k) { return k > 100 ? 100 : (k < -100 ? -100 : k); };
+            if (!MAPS) {
                 int rank = 0;
                 for (int b = 0; b < nl && rank < r1; b += 32) {
                     double iv, sv; float wm; int ew;
                     group(b, iv, sv, wm, ew);
                     const unsigned bal = __ballot_sync(FULL, iv != 0.0);
                     const int my = rank + __popc(bal & ((1u << lane) - 1u));
-                    if (iv != 0.0 && my >= r0 && my < r1) {
-                        const double s = fmax(sv, 1e-9);
-                        const double bnd = fabs(iv) * kInv2Pi / (s * s) * (double)wm *
-                                           (1.0 + 2.5066282746310002 * s / J.dsx);
-                        int q = 0;
-                        if (bnd > 0.0 && bnd < 1e300) {
-                            (void)frexp(bnd, &q);          // bnd < 2^q
-                            ks = min(ks, 14 - q);
-                        }
-                    }
+                    if (iv != 0.0 && my >= r0 && my < r1) ks = min(ks, scale(iv, fmax(sv, 1e-9), wm));
                     rank += __popc(bal);
                 }
-                ks = __reduce_min_sync(FULL, ks);
-                ks = ks > 100 ? 100 : (ks < -100 ? -100 : ks);
+                ks = clamp(__reduce_min_sync(FULL, ks));
             }
             const int tyy = tile / J.ntx, txx = tile % J.ntx;
             const int sym = (P.sym && tyy == txx) ? kSym : 0;
@@ -378,6 +383,7 @@ __device__ __forceinline__ void scheduler_warp(const Params& P, uint8_t* smem, S
                 if (mine) {
                     const int l = b + lane;
                     const double s = fmax(sv, 1e-9);
+                    if (MAPS) ks = clamp(scale(iv, s, wm));   // every step is its own output
                     st.job = job; st.z = z; st.tile = tile; st.l = l;
                     st.chunk = c; st.nch = nch;
                     st.flags = (my == r0 ? kFirst | kTab : 0) | (my == r1 - 1 ? kLast : 0) | sym;
@@ -470,6 +476,7 @@ __device__ __forceinline__ void issue2(uint32_t d, uint32_t a, uint32_t b, uint3
     }
 }
 
+template <bool MAPS>
 __device__ __forceinline__ void mma_warp(const Params& P, uint32_t sbase, uint32_t tb, int role,
                                          const Step* ring, uint64_t* full, uint64_t* empty,
                                          const Bars& B) {
@@ -527,8 +534,11 @@ __device__ __forceinline__ void mma_warp(const Params& P, uint32_t sbase, uint32
             if (lane == 0) {
                 const uint32_t a = sbase + P.oA2 + (uint32_t)ia * 2u * aBytes2;
                 const uint32_t b = sbase + P.oB2 + (uint32_t)ib * 2u * aBytes2;
-                issue2(role == 2 ? tb + kColDb + (uint32_t)db * 128u : tb + kColDc, a, b, aBytes2, N1 / 16,
-                       id2, role == 2 || first ? 0u : 1u, role == 3);
+                const uint32_t d = role == 2 ? tb + kColDb + (uint32_t)db * 128u : tb + kColDc;
+                // maps: the step's cross products first, so that only the hi * hi products
+                // accumulate on large values
+                if (MAPS) issue2(d, a, b, aBytes2, N1 / 16, id2, 0u, true);
+                issue2(d, a, b, aBytes2, N1 / 16, id2, MAPS || (role == 3 && !first) ? 1u : 0u, role == 3);
                 if (role == 2) tc::commit(&B.df[db]);
                 tc::commit(&B.a2f[ia]);
                 tc::commit(&B.b2f[ib]);
@@ -551,6 +561,7 @@ __device__ __forceinline__ void mma_warp(const Params& P, uint32_t sbase, uint32
 // ------------------------------------------------------------------------------------------
 // Math warps.
 // ------------------------------------------------------------------------------------------
+template <bool MAPS>
 __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint32_t tb,
                                            const Step* ring, uint64_t* full, uint64_t* empty,
                                            const Bars& B) {
@@ -727,6 +738,40 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
         return true;
     };
 
+    // Maps: this warp's 32 rows x 64 columns of one layer's map, TMEM -> global memory, whole
+    // sectors (a lane's stores are 32 bytes wide where the rows allow it: 16-byte ones half fill
+    // each sector they touch).
+    auto map_rows = [&](const Step& st, float sc, uint32_t col) {
+        const JobDev& J = P.jobs[st.job];
+        const int ty = st.tile / J.ntx, tx = st.tile % J.ntx;
+        const int y = ty * kTile + trow, xb = tx * kTile + half * 64;
+        float* d = J.dose + (size_t)st.l * J.layer_stride + ((size_t)st.z * J.ny + y) * J.nx + xb;
+        const int left = y < J.ny ? J.nx - xb : 0;
+        const bool wide = (J.nx & 7) == 0 && ((size_t)d & 31) == 0;
+#pragma unroll 1
+        for (int c = 0; c < 64; c += 16) {
+            uint32_t r[16];
+            tc::tmem_ld16(col + (uint32_t)c, r);
+            tc::tmem_wait_ld();
+            float v[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(r[q]) * sc;
+            if (wide) {
+#pragma unroll
+                for (int q = 0; q < 16; q += 8)
+                    if (c + q < left)
+                        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(d + c + q),
+                                     "f"(v[q]), "f"(v[q + 1]), "f"(v[q + 2]), "f"(v[q + 3]), "f"(v[q + 4]),
+                                     "f"(v[q + 5]), "f"(v[q + 6]), "f"(v[q + 7])
+                                     : "memory");
+            } else {
+#pragma unroll
+                for (int q = 0; q < 16; ++q)
+                    if (c + q < left) d[c + q] = v[q];
+            }
+        }
+    };
+
     // DR: step m's hi * hi product into dsum; at its unit's end the cross products and output.
     auto dr = [&](const Step& st, int m) -> bool {
         const int db = m & 1;
@@ -735,37 +780,44 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
         tc::fence_after_sync();
         const float sc = __int_as_float((127 - st.kd) << 23);   // 2^-kd, exact (|kd| <= 114)
         const f32x2 sc2 = pk(sc, sc);
-        uint32_t r[4][16];
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-            tc::tmem_ld16(tb + kColDb + (uint32_t)db * 128u + lane_base + (uint32_t)(half * 64 + c * 16), r[c]);
-        tc::tmem_wait_ld();
-        tc::fence_before_sync();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&B.du[db]);
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-                dsum[c * 8 + q] = fma2(pk(__uint_as_float(r[c][2 * q]), __uint_as_float(r[c][2 * q + 1])), sc2, dsum[c * 8 + q]);
-        if (st.flags & kLast) {
-            w = wait_bar(B.cf, (uint32_t)(useg & 1), P.wait_ns);
-            if (!__all_sync(0xffffffffu, w)) return false;
-            tc::fence_after_sync();
+        if constexpr (MAPS) {
+            map_rows(st, sc, tb + kColDb + (uint32_t)db * 128u + lane_base + (uint32_t)(half * 64));
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&B.du[db]);
+        } else {
+            uint32_t r[4][16];
 #pragma unroll
             for (int c = 0; c < 4; ++c)
-                tc::tmem_ld16(tb + kColDc + lane_base + (uint32_t)(half * 64 + c * 16), r[c]);
+                tc::tmem_ld16(tb + kColDb + (uint32_t)db * 128u + lane_base + (uint32_t)(half * 64 + c * 16), r[c]);
             tc::tmem_wait_ld();
             tc::fence_before_sync();
             __syncwarp();
-            if (lane == 0) tc::mbar_arrive(B.cu);
-            ++useg;
+            if (lane == 0) tc::mbar_arrive(&B.du[db]);
 #pragma unroll
             for (int c = 0; c < 4; ++c)
 #pragma unroll
                 for (int q = 0; q < 8; ++q)
                     dsum[c * 8 + q] = fma2(pk(__uint_as_float(r[c][2 * q]), __uint_as_float(r[c][2 * q + 1])), sc2, dsum[c * 8 + q]);
-            output(st, false);
+            if (st.flags & kLast) {
+                w = wait_bar(B.cf, (uint32_t)(useg & 1), P.wait_ns);
+                if (!__all_sync(0xffffffffu, w)) return false;
+                tc::fence_after_sync();
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    tc::tmem_ld16(tb + kColDc + lane_base + (uint32_t)(half * 64 + c * 16), r[c]);
+                tc::tmem_wait_ld();
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(B.cu);
+                ++useg;
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        dsum[c * 8 + q] = fma2(pk(__uint_as_float(r[c][2 * q]), __uint_as_float(r[c][2 * q + 1])), sc2, dsum[c * 8 + q]);
+                output(st, false);
+            }
         }
         return true;
     };
@@ -827,6 +879,8 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
     if (!ok && lane == 0) atomicExch(P.err, 1);
 }
 
+// MAPS: per-layer maps (jobs with layer_stride > 0): every step's map is its own output.
+template <bool MAPS>
 __global__ void __launch_bounds__(kThreads, 1) fwd_tc16_kernel(Params P) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[kRing];
@@ -844,7 +898,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_tc16_kernel(Params P) {
     if (threadIdx.x == 0) {
         for (int i = 0; i < kRing; ++i) {
             tc::mbar_init(&full[i], 1);
-            tc::mbar_init(&empty[i], kMathWarps + 3);   // math warps + the three MMA warps
+            tc::mbar_init(&empty[i], kMathWarps + (MAPS ? 2 : 3));   // math and MMA warps
         }
         for (int i = 0; i < 4; ++i) {
             tc::mbar_init(&B.wfull[i], 1);             // producer's expect_tx arrival + bytes
@@ -852,13 +906,13 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_tc16_kernel(Params P) {
         }
         for (int i = 0; i < 3; ++i) {
             tc::mbar_init(&B.a2r[i], kMathWarps);
-            tc::mbar_init(&B.a2f[i], 3);               // stage 1 and both stage-2 warps
+            tc::mbar_init(&B.a2f[i], MAPS ? 2 : 3);    // stage 1 and the stage-2 warps
         }
         for (int i = 0; i < 2; ++i) {
             tc::mbar_init(&B.a1r[i], kMathWarps);
             tc::mbar_init(&B.a1f[i], 1);
             tc::mbar_init(&B.b2r[i], kMathWarps);
-            tc::mbar_init(&B.b2f[i], 2);
+            tc::mbar_init(&B.b2f[i], MAPS ? 1 : 2);
             tc::mbar_init(&B.df[i], 1);
             tc::mbar_init(&B.du[i], kMathWarps);
         }
@@ -882,12 +936,12 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_tc16_kernel(Params P) {
     if (warp >= kMathWarps) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kCtrlRegs));
         if (warp == kSchedWarp)
-            scheduler_warp(P, smem, ring, full, empty, B.wfull, B.wempty);
-        else
-            mma_warp(P, tc::smem_u32(smem), tmem_base_s, warp - kSchedWarp, ring, full, empty, B);
+            scheduler_warp<MAPS>(P, smem, ring, full, empty, B.wfull, B.wempty);
+        else if (!MAPS || warp != kS3Warp)   // maps: one warp issues all of stage 2
+            mma_warp<MAPS>(P, tc::smem_u32(smem), tmem_base_s, warp - kSchedWarp, ring, full, empty, B);
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kMathRegs));
-        math_warps(P, smem, tmem_base_s, ring, full, empty, B);
+        math_warps<MAPS>(P, smem, tmem_base_s, ring, full, empty, B);
     }
 
     tc::fence_before_sync();
@@ -1099,7 +1153,12 @@ int launch_forward_tc16(JobDev* jobs_dev, const JobDev* jobs_host, int n_jobs, i
         nsx = std::max(nsx, jobs_host[j].nsx);
         nsy = std::max(nsy, jobs_host[j].nsy);
     }
-    if (jobs_host[0].layer_stride != 0) return PBD_ERR_UNSUPPORTED;   // per-layer maps: TF32 kernel
+    // per-layer maps (layer_stride > 0, no loss) or the dose: every job of a launch alike
+    const bool maps = jobs_host[0].layer_stride != 0;
+    for (int j = 1; j < n_jobs; ++j)
+        if ((jobs_host[j].layer_stride != 0) != maps) return PBD_ERR_UNSUPPORTED;
+    if (maps && (with_loss || poison)) return PBD_ERR_UNSUPPORTED;
+    auto* kernel = maps ? fwd_tc16_kernel<true> : fwd_tc16_kernel<false>;
     P.sym = 1;
     for (int j = 0; j < n_jobs; ++j) {
         const JobDev& J = jobs_host[j];
@@ -1119,7 +1178,7 @@ int launch_forward_tc16(JobDev* jobs_dev, const JobDev* jobs_host, int n_jobs, i
     P.wmax = wmax;
     P.wexp = wexp;
     int max_dyn = 0;
-    PBD_TRY(smem_optin((const void*)fwd_tc16_kernel, -1, kLaunchRegsNeeded, &max_dyn));
+    PBD_TRY(smem_optin((const void*)kernel, -1, kLaunchRegsNeeded, &max_dyn));
     Plan16 pl;
     if (!plan16(P.K1, P.N1, max_dyn, &pl)) return PBD_ERR_NO_SMEM;
     P.nR = pl.nR; P.nA1 = pl.nA1; P.nA2 = pl.nA2; P.nB2 = pl.nB2;
@@ -1140,9 +1199,10 @@ int launch_forward_tc16(JobDev* jobs_dev, const JobDev* jobs_host, int n_jobs, i
                              inst ? 1 : 0, inst_dst, inst_status));
     const int grid = std::max(1, std::min(P.n_units, num_sms()));
     prof_mark(kProfFwd, 0, s);
-    PBD_TRY(launch_dependent(fwd_tc16_kernel, dim3(grid), dim3(kThreads), smem, s, P));
+    PBD_TRY(launch_dependent(kernel, dim3(grid), dim3(kThreads), smem, s, P));
     prof_mark(kProfFwd, 1, s);
     count_launch(2);
+    if (maps) return PBD_OK;   // the caller reads the error word
     // every job of a launch shares its output mode (the callers set it per launch)
     if (!jobs_host[0].direct || with_loss) {
         size_t maxn = 1;
