@@ -19,14 +19,15 @@
 // Kernels (all on `stream`, no host synchronisation):
 //   gamma_refmax_kernel   max of the reference dose (skipped when a normalisation dose is given)
 //   gamma_kernel          one thread per 4 voxels along z, the evaluated dose of a 32x8x4 brick
-//                         plus its halo staged in shared memory as FP64; offsets visited in
-//                         ascending (|o|/DTA)^2, stopping once that weight reaches the current
-//                         minimum (exact: w + d^2 >= w after rounding); masked voxels' gamma
+//                         plus its halo staged in shared memory; a screen in the doses' own type
+//                         with the reciprocal criterion finds the smallest sum over the offsets
+//                         (in ascending (|o|/DTA)^2, stopping once that weight exceeds the
+//                         minimum), which alone is then formed exactly; masked voxels' gamma
 //                         appended to a key list; per-block partial sums and maxima
 //   (same kernel, fallback pass: runs only when the threshold mask was empty)
 //   gamma_finish_kernel   counts, mean, max, pass rate, percentile ranks (NumPy 'linear')
-//   gamma_select_kernel   radix select of the four order statistics the percentiles need (one
-//                         launch per digit; the last block to arrive picks the digits)
+//   gamma_select_kernel   radix select of the four order statistics the percentiles need (the
+//                         last block to arrive picks a digit; one block finishes the candidates)
 //   gamma_final_kernel    NumPy's interpolation between the order statistics
 #include <math.h>
 #include <string.h>
@@ -53,7 +54,7 @@ constexpr int kRowBatch = 4;           // staged rows per warp whose loads are i
 // largest staged brick (radius 6 on every axis) and offset list (13^3 offsets)
 constexpr int kGMaxOff = 13 * 13 * 13;
 constexpr int kGMaxSmem = (kTX + 12) * (kTY + 12) * (kTZ + 12) * (int)sizeof(double) +
-                          kGMaxOff * (int)(sizeof(double) + sizeof(int));
+                          kGMaxOff * (int)(2 * sizeof(double) + sizeof(int));
 
 struct GammaParams {
     int nz, ny, nx;
@@ -88,6 +89,7 @@ struct GammaState {
     unsigned long long n_eval, n_pass, n_nan;
     unsigned int sel_arrive;           // blocks of the current select pass that finished
     unsigned long long n_cand;         // keys copied to the candidate list
+    int sel_done;                      // the select passes are complete
 };
 
 // Order-preserving map of a double to an unsigned key (NaN above +inf).
@@ -105,7 +107,6 @@ __device__ __forceinline__ double nmin(double a, double b) {
     if (a != a || b != b) return __longlong_as_double(0x7FF8000000000000ll);
     return b < a ? b : a;
 }
-__device__ __forceinline__ bool finite_d(double v) { return v == v && v - v == 0.0; }
 
 template <class T>
 __device__ __forceinline__ double ld(const T* p, size_t i) { return (double)__ldg(p + i); }
@@ -127,18 +128,38 @@ gamma_refmax_kernel(const T* __restrict__ ref, size_t n, GammaState* st) {
     if ((threadIdx.x & 31) == 0 && best) atomicMax(&st->ref_key, best);
 }
 
+// Doses and criteria inside [1 / kTame, kTame] in magnitude go through the screen: nothing overflows
+// in it that would not make the sum larger than the smallest.  Others (and tiles with any other dose,
+// infinities and NaN included) take every offset's exact sum.
+constexpr double kTame = 1e30;
+// Relative width that separates sums for certain: the screen's own error is below 4 roundings of q,
+// twice that in q^2, and one of the weight and of the sum (10 units of 2^-24 or 2^-53).
+template <class T> struct Screen;
+template <> struct Screen<float> { static constexpr float rel = 0x1p-18f; };
+template <> struct Screen<double> { static constexpr double rel = 0x1p-46; };
+
+__device__ __forceinline__ double local_crit(const GammaParams& P, double r, double crit_g) {
+    return P.local ? __dmul_rn(P.crit_frac, r > 1e-12 || r != r ? r : 1e-12) : crit_g;
+}
+
+// Doubles that the offset tables (weights in FP64 and in T, positions) take before the tile.
+template <class T>
+constexpr __host__ __device__ size_t gamma_offset_doubles(int n_off) {
+    return ((size_t)n_off * (sizeof(double) + sizeof(T) + sizeof(int)) + 7) / 8;
+}
+
 template <class T, bool kFallback>
-__global__ void __launch_bounds__(kGThreads)
+__global__ void __launch_bounds__(kGThreads, sizeof(T) == 4 ? 4 : 3)
 gamma_kernel(const GammaParams P, const T* __restrict__ ref, const T* __restrict__ ev,
              double* __restrict__ gmap, unsigned char* __restrict__ mmap, GammaState* st,
              unsigned long long* __restrict__ keys, double* __restrict__ part_sum,
              double* __restrict__ part_max, int gx, int gy, int n_bricks) {
-    extern __shared__ double tile[];
+    extern __shared__ double smem[];
     __shared__ double red_s[kGThreads / 32], red_m[kGThreads / 32];
-    __shared__ unsigned long long red_c[kGThreads / 32][3];
+    __shared__ unsigned red_c[kGThreads / 32][3];
     __shared__ unsigned int s_wcnt[kGThreads / 32], s_wpre[kGThreads / 32];
     __shared__ unsigned long long s_base;
-    __shared__ int s_nonfinite;
+    __shared__ int s_wild;
     const int pass = kFallback ? 1 : 0;
     if (kFallback && __ldcg(&st->cnt[0][0]) != 0ull) return;   // the threshold mask is used
     const double ref_max = P.use_ref_dose ? P.ref_dose : dunkey(__ldcg(&st->ref_key));
@@ -149,8 +170,11 @@ gamma_kernel(const GammaParams P, const T* __restrict__ ref, const T* __restrict
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int TX = kTX + 2 * P.hx, TY = kTY + 2 * P.hy, TZ = kTZ + 2 * P.hz;
     const int plane = TX * TY;
-    double* s_w = tile + (size_t)plane * TZ;                    // weight of each offset
-    int* s_off = reinterpret_cast<int*>(s_w + P.n_off);         // its position in the tile
+    const int inv_ty = (65536 + TY - 1) / TY;                    // row / TY for the tile's rows (<= 320)
+    double* s_w = smem;                                         // weight of each offset
+    T* s_wt = reinterpret_cast<T*>(s_w + P.n_off);              // the same, for the screen
+    int* s_off = reinterpret_cast<int*>(s_wt + P.n_off);        // its position in the tile
+    T* tile = reinterpret_cast<T*>(smem + gamma_offset_doubles<T>(P.n_off));
     // offsets of each (|a|,|b|,|c|) entry with their signs, in ascending weight
     for (int u = tid; u < P.n_entries; u += kGThreads) {
         const int ia = P.abc[u][0], ib = P.abc[u][1], ic = P.abc[u][2];
@@ -160,103 +184,150 @@ gamma_kernel(const GammaParams P, const T* __restrict__ ref, const T* __restrict
                 continue;
             const int sa = (sgn & 4) ? -ia : ia, sb = (sgn & 2) ? -ib : ib, sc = (sgn & 1) ? -ic : ic;
             s_w[o] = P.w[u];
+            s_wt[o] = (T)P.w[u];
             s_off[o] = sa * plane + sb * TX + sc;
             ++o;
         }
     }
     const double crit_g = __dmul_rn(P.crit_frac, ref_max);     // global dose criterion
     const double thr_dose = __dmul_rn(P.thr_frac, ref_max);
-    const bool ok_g = finite_d(crit_g) || P.local;
     const int tx = lane, ty = warp;
     double sum = 0.0, mx = -1.0;                 // gamma >= 0
-    unsigned long long c_eval = 0, c_pass = 0, c_nan = 0;
+    unsigned c_eval = 0, c_pass = 0, c_nan = 0;
     // bricks of 32 x 8 x 4 voxels, statically strided over the persistent blocks
     for (int brick = blockIdx.x; brick < n_bricks; brick += gridDim.x) {
         const int bx = brick % gx, rest = brick / gx, by = rest % gy, bz = rest / gy;
         const int x0 = bx * kTX, y0 = by * kTY, z0 = bz * kTZ;
         const int x = x0 + tx, y = y0 + ty;
         // this thread's reference doses, loaded before the staging barrier
-        double rv[kTZ];
+        T rv[kTZ];
 #pragma unroll
         for (int k = 0; k < kTZ; ++k) {
             const int z = z0 + k;
             rv[k] = (x < P.nx && y < P.ny && z < P.nz)
-                        ? ld(ref, ((size_t)z * P.ny + y) * P.nx + x) : 0.0;
+                        ? __ldg(ref + ((size_t)z * P.ny + y) * P.nx + x) : T(0);
         }
         __syncthreads();                         // the previous brick is done with the tile
-        if (tid == 0) s_nonfinite = 0;
+        if (tid == 0) s_wild = 0;
         __syncthreads();
         // the evaluated dose of the brick and its halo: each warp takes rows of TX voxels,
         // kRowBatch rows' loads issued before their stores
-        int nonfin = 0;
+        bool wild = false;
         const int n_rows = TY * TZ;
+        auto load = [&](int row, int col) -> T {
+            const int tz = (row * inv_ty) >> 16, tyy = row - tz * TY;
+            const int z = z0 - P.hz + tz, yy = y0 - P.hy + tyy, xx = x0 - P.hx + col;
+            const bool ok = row < n_rows && z >= 0 && z < P.nz && yy >= 0 && yy < P.ny && xx >= 0 && xx < P.nx;
+            return ok ? __ldg(ev + ((size_t)z * P.ny + yy) * P.nx + xx) : T(0);
+        };
         for (int row0 = warp; row0 < n_rows; row0 += kRowBatch * (kGThreads / 32)) {
-            for (int t0 = 0; t0 < TX; t0 += 32) {
-                double v[kRowBatch];
+            T v[kRowBatch];
 #pragma unroll
-                for (int q = 0; q < kRowBatch; ++q) {
-                    const int row = row0 + q * (kGThreads / 32);
-                    const int tz = row / TY, tyy = row - tz * TY;
-                    const int z = z0 - P.hz + tz, yy = y0 - P.hy + tyy, xx = x0 - P.hx + t0 + lane;
-                    const bool ok = row < n_rows && t0 + lane < TX && z >= 0 && z < P.nz &&
-                                    yy >= 0 && yy < P.ny && xx >= 0 && xx < P.nx;
-                    v[q] = ok ? ld(ev, ((size_t)z * P.ny + yy) * P.nx + xx) : 0.0;
-                }
+            for (int q = 0; q < kRowBatch; ++q) v[q] = load(row0 + q * (kGThreads / 32), P.hx + lane);
 #pragma unroll
-                for (int q = 0; q < kRowBatch; ++q) {
-                    const int row = row0 + q * (kGThreads / 32);
-                    if (row < n_rows && t0 + lane < TX) {
-                        nonfin |= !finite_d(v[q]);
-                        tile[row * TX + t0 + lane] = v[q];
-                    }
-                }
+            for (int q = 0; q < kRowBatch; ++q) {
+                const int row = row0 + q * (kGThreads / 32);
+                wild |= !(fabs((double)v[q]) <= kTame);
+                if (row < n_rows) tile[row * TX + P.hx + lane] = v[q];
             }
         }
-        if (nonfin) s_nonfinite = 1;
+        // the halo's columns, both sides of a row together
+        for (int e = tid; e < n_rows * 2 * P.hx; e += kGThreads) {
+            const int row = e / (2 * P.hx), c = e - row * 2 * P.hx, col = c < P.hx ? c : kTX + c;
+            const T v = load(row, col);
+            wild |= !(fabs((double)v) <= kTame);
+            tile[row * TX + col] = v;
+        }
+        if (wild) s_wild = 1;
         __syncthreads();
-        const bool tile_finite = s_nonfinite == 0;
-        double gk[kTZ];
+        const bool tame = s_wild == 0;
+        // the voxels whose gamma is needed: the masked ones, all of them for a gamma map
+        const size_t v0 = ((size_t)z0 * P.ny + y) * P.nx + x, nslice = (size_t)P.ny * P.nx;
+        const T* c0 = tile + (size_t)P.hz * plane + (ty + P.hy) * TX + (tx + P.hx);
+        unsigned need = 0, msk = 0, screened = 0;
+        T inv[kTZ], a1[kTZ], a2[kTZ];
+        int jb[kTZ];
+#pragma unroll
+        for (int k = 0; k < kTZ; ++k) {
+            const bool in = x < P.nx && y < P.ny && z0 + k < P.nz;
+            const double r = rv[k];
+            const bool m = in && (kFallback ? (r > 0.0) : (r >= thr_dose));
+            const bool n = m || (in && !kFallback && P.want_gamma);
+            const double crit = local_crit(P, r, crit_g);
+            const bool ok = n && tame && fabs(r) <= kTame && fabs(crit) <= kTame && fabs(crit) >= 1.0 / kTame;
+            msk |= m ? 1u << k : 0u;
+            need |= n ? 1u << k : 0u;
+            screened |= ok ? 1u << k : 0u;
+            inv[k] = T(1) / (T)crit;
+            a1[k] = ok ? T(INFINITY) : -T(INFINITY);
+            a2[k] = T(INFINITY);
+            jb[k] = 0;
+        }
+        // Dividing out every offset (FP64 division and square root, 860 instructions per 32 voxels at 19
+        // offsets, blocks that strode over the bricks) took 81 us at 128^3, now 50: instruction issue,
+        // a third of it the screen, a fifth the exact sums and square roots.
+        // The screen: the smallest and the second smallest sum in T with the reciprocal of the
+        // criterion, both within kScreen of the sum the exact operations give.
+        for (int j = 0; j < P.n_off; ++j) {
+            const T w = s_wt[j];
+            const T worst = fmax(fmax(a1[0], a1[1]), fmax(a1[2], a1[3]));
+            if (w > worst + worst * Screen<T>::rel) break;
+            const T* c = c0 + s_off[j];
+#pragma unroll
+            for (int k = 0; k < kTZ; ++k) {
+                const T q = (c[k * plane] - rv[k]) * inv[k];
+                const T a = fma(q, q, w);
+                a2[k] = fmin(a2[k], fmax(a1[k], a));
+                jb[k] = a < a1[k] ? j : jb[k];
+                a1[k] = fmin(a1[k], a);
+            }
+        }
+        // The exact sum of the smallest; voxels where another sum may be as small (or that the screen
+        // does not cover) take every offset's, one voxel at a time.
+        double best[kTZ] = {};
+        unsigned rare = 0;
+        auto exact = [&](int k, int j, double r, double crit) {
+            const double dd = __ddiv_rn(__dsub_rn((double)c0[k * plane + s_off[j]], r), crit);
+            return __dadd_rn(s_w[j], __dmul_rn(dd, dd));
+        };
+#pragma unroll
+        for (int k = 0; k < kTZ; ++k) {
+            if (!((need >> k) & 1u)) continue;
+            best[k] = exact(k, jb[k], rv[k], local_crit(P, rv[k], crit_g));
+            const bool only = ((screened >> k) & 1u) && a2[k] > a1[k] + a1[k] * Screen<T>::rel;
+            rare |= only ? 0u : 1u << k;
+        }
+        while (rare) {
+            const int k = __ffs(rare) - 1;
+            rare &= rare - 1u;
+            const double r = ld(ref, v0 + k * nslice), crit = local_crit(P, r, crit_g);
+            const bool stop = (screened >> k) & 1u;
+            double m = __longlong_as_double(0x7FF0000000000000ll);    // +inf
+            for (int j = 0; j < P.n_off; ++j) {
+                if (stop && s_w[j] >= m) break;      // w + d^2 >= w >= m, here and later
+                m = nmin(m, exact(k, j, r, crit));
+            }
+#pragma unroll
+            for (int q = 0; q < kTZ; ++q) best[q] = q == k ? m : best[q];
+        }
         unsigned int bal[kTZ];
         unsigned int wcnt = 0;
 #pragma unroll
         for (int k = 0; k < kTZ; ++k) {
-            const int z = z0 + k;
-            const bool in = x < P.nx && y < P.ny && z < P.nz;
+            const bool masked = (msk >> k) & 1u;
             double g = 0.0;
-            bool masked = false;
-            if (in) {
-                const size_t v = ((size_t)z * P.ny + y) * P.nx + x;
-                const double r = rv[k];
-                masked = kFallback ? (r > 0.0) : (r >= thr_dose);
-                // without a gamma map only masked voxels need their gamma
-                if (masked || (!kFallback && P.want_gamma)) {
-                    const double crit =
-                        P.local ? __dmul_rn(P.crit_frac, r > 1e-12 || r != r ? r : 1e-12) : crit_g;
-                    // early exit is exact when no NaN can appear later: finite doses, a finite
-                    // non-zero criterion (NaN needs 0/0, inf - inf or inf/inf)
-                    const bool fast =
-                        tile_finite && finite_d(r) && finite_d(crit) && crit != 0.0 && ok_g;
-                    const double* c0 =
-                        tile + (size_t)(k + P.hz) * plane + (ty + P.hy) * TX + (tx + P.hx);
-                    double best = __longlong_as_double(0x7FF0000000000000ll);    // +inf
-                    for (int j = 0; j < P.n_off; ++j) {
-                        const double w = s_w[j];
-                        if (fast && w >= best) break;    // w + d^2 >= w >= best, here and later
-                        const double dd = __ddiv_rn(__dsub_rn(c0[s_off[j]], r), crit);
-                        best = nmin(best, __dadd_rn(w, __dmul_rn(dd, dd)));
-                    }
-                    g = __dsqrt_rn(best);
-                    if (!kFallback && P.want_gamma) gmap[v] = g;
-                }
-                if (P.want_mask) mmap[v] = masked ? 1 : 0;
+            if ((need >> k) & 1u) {
+                g = __dsqrt_rn(best[k]);
+                if (!kFallback && P.want_gamma) gmap[v0 + k * nslice] = g;
             }
+            if (P.want_mask && x < P.nx && y < P.ny && z0 + k < P.nz) mmap[v0 + k * nslice] = masked ? 1 : 0;
             if (masked) {
                 ++c_eval;
                 c_pass += g <= 1.0;
                 if (g != g) ++c_nan;
                 else { sum = __dadd_rn(sum, g); mx = g > mx ? g : mx; }
             }
-            gk[k] = g;
+            best[k] = g;
             bal[k] = __ballot_sync(0xffffffffu, masked);
             wcnt += __popc(bal[k]);
         }
@@ -273,7 +344,7 @@ gamma_kernel(const GammaParams P, const T* __restrict__ ref, const T* __restrict
         const unsigned int below = (1u << lane) - 1u;
 #pragma unroll
         for (int k = 0; k < kTZ; ++k) {
-            if (bal[k] & (1u << lane)) keys[pos + __popc(bal[k] & below)] = dkey(gk[k]);
+            if (bal[k] & (1u << lane)) keys[pos + __popc(bal[k] & below)] = dkey(best[k]);
             pos += __popc(bal[k]);
         }
     }
@@ -359,141 +430,165 @@ gamma_finish_kernel(const GammaParams P, GammaState* st, const double* __restric
     for (int j = 0; j < 4; ++j) { st->prefix[j] = 0ull; st->rem[j] = st->rank[j]; }
 }
 
-// One radix-select pass over key bits [shift, top) (digits of 11 bits from the top, the last
-// one 9 bits).  The blocks histogram the keys whose bits above `top` equal a target's prefix
-// (targets with equal prefixes share a histogram; runs of equal digits are counted in
-// registers before one shared-memory atomic), add their histograms to the global one, and
-// the last block to arrive picks each target's digit from the totals, updates its prefix and
-// remaining rank, and clears the histogram and the arrival counter for the next pass.
-// mode 0 reads every masked key; mode 1 also copies the keys that match any target's
-// prefix into a candidate list; mode 2 reads only the candidates.  The grid is trimmed to
-// about kSelPer keys per thread.
+// Radix select: passes over key bits [shift, top) (digits of 11 bits from the top, the last one 9
+// bits).  The blocks histogram the keys whose bits above `top` equal a target's prefix (targets
+// with equal prefixes share a histogram; runs of equal digits are counted in registers before one
+// shared-memory atomic), add their histograms to the global one, and the last block to arrive picks
+// each target's digit from the totals, updates its prefix and remaining rank, and clears the
+// histogram and the arrival counter for the next pass.
+// mode 0 reads every masked key; mode 1 also copies the keys that match any target's prefix into a
+// candidate list; mode 2 reads only the candidates.  The grid is trimmed to about kSelPer keys per
+// thread; once one block is enough for the candidates (nearly always), it takes all the passes that
+// are left without the global histogram, and the launches after it have nothing to do.
+// 128^3: six passes of 11 us with a bin scan that conflicted on one bank, together
+// 57 us now.
 __global__ void __launch_bounds__(kHistThreads)
 gamma_select_kernel(GammaState* st, const unsigned long long* __restrict__ keys,
-                    unsigned long long* __restrict__ cand, int shift, int top, int mode,
+                    unsigned long long* __restrict__ cand, int pass, int mode,
                     unsigned int* __restrict__ hist) {
     __shared__ unsigned int h[4][kBins];
     __shared__ int s_last;
-    if (st->status != 0) return;
+    if (st->status != 0 || st->sel_done) return;
     const unsigned long long n = mode == 2 ? st->n_cand : st->n_eval;
     const unsigned long long* src = mode == 2 ? cand : keys;
     const unsigned long long want = (n + (unsigned long long)kHistThreads * kSelPer - 1) /
                                     ((unsigned long long)kHistThreads * kSelPer);
     const unsigned int active = (unsigned int)(want < gridDim.x ? (want ? want : 1) : gridDim.x);
     if (blockIdx.x >= active) return;
-    const unsigned long long himask = top >= 64 ? 0ull : ~((1ull << top) - 1ull);
-    const unsigned int dmask = (1u << (top - shift)) - 1u;
-    unsigned long long pre[4];
-    int grp[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        pre[j] = st->prefix[j];
-        grp[j] = j;
-        for (int q = 0; q < j; ++q)
-            if (grp[j] == j && pre[q] == pre[j]) grp[j] = grp[q];
-    }
-    for (int j = 0; j < 4; ++j)
-        if (grp[j] == j)
-            for (int i = threadIdx.x; i < kBins; i += kHistThreads) h[j][i] = 0u;
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    unsigned int rd[4] = {0u, 0u, 0u, 0u}, rc[4] = {0u, 0u, 0u, 0u};
-    const unsigned long long stride = (unsigned long long)active * kHistThreads;
-    // warp-uniform trip count (the candidate append is warp-collective); four keys per
-    // thread loaded before they are counted
-    for (unsigned long long b0 = (unsigned long long)blockIdx.x * kHistThreads + (threadIdx.x & ~31);
-         b0 < n; b0 += 4 * stride) {
-      unsigned long long kk[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const unsigned long long i = b0 + q * stride + lane;
-        kk[q] = i < n ? __ldg(src + i) : 0ull;
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const unsigned long long b = b0 + q * stride;
-        if (b >= n) break;                                   // warp-uniform
-        const bool valid = b + lane < n;
-        const unsigned long long k = kk[q];
-        const unsigned int d = (unsigned int)(k >> shift) & dmask;
-        bool any = false;
+    const bool alone = mode == 2 && active == 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int p = pass; p < (alone ? kSelPasses : pass + 1); ++p) {
+        const int top = 64 - kDigitBits * p;                       // 64, 53, 42, 31, 20, 9
+        const int shift = top > kDigitBits ? top - kDigitBits : 0;
+        const unsigned long long himask = top >= 64 ? 0ull : ~((1ull << top) - 1ull);
+        const unsigned int dmask = (1u << (top - shift)) - 1u;
+        unsigned long long pre[4];
+        int grp[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            if (grp[j] != j || !valid || (k & himask) != pre[j]) continue;
-            any = true;
-            if (rc[j] && rd[j] == d) { ++rc[j]; continue; }
+            pre[j] = __ldcg(&st->prefix[j]);
+            grp[j] = j;
+            for (int q = 0; q < j; ++q)
+                if (grp[j] == j && pre[q] == pre[j]) grp[j] = grp[q];
+        }
+        for (int j = 0; j < 4; ++j)
+            if (grp[j] == j)
+                for (int i = threadIdx.x; i < kBins; i += kHistThreads) h[j][i] = 0u;
+        __syncthreads();
+        unsigned int rd[4] = {0u, 0u, 0u, 0u}, rc[4] = {0u, 0u, 0u, 0u};
+        const unsigned long long stride = (unsigned long long)active * kHistThreads;
+        // warp-uniform trip count (the candidate append is warp-collective); four keys per
+        // thread loaded before they are counted
+        for (unsigned long long b0 = (unsigned long long)blockIdx.x * kHistThreads + (threadIdx.x & ~31);
+             b0 < n; b0 += 4 * stride) {
+            unsigned long long kk[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const unsigned long long i = b0 + q * stride + lane;
+                kk[q] = i < n ? __ldg(src + i) : 0ull;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const unsigned long long b = b0 + q * stride;
+                if (b >= n) break;                                   // warp-uniform
+                const bool valid = b + lane < n;
+                const unsigned long long k = kk[q];
+                const unsigned int d = (unsigned int)(k >> shift) & dmask;
+                bool any = false;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (grp[j] != j || !valid || (k & himask) != pre[j]) continue;
+                    any = true;
+                    if (rc[j] && rd[j] == d) { ++rc[j]; continue; }
+                    if (rc[j]) atomicAdd(&h[j][rd[j]], rc[j]);
+                    rd[j] = d;
+                    rc[j] = 1u;
+                }
+                if (mode == 1) {
+                    const unsigned int bal = __ballot_sync(0xffffffffu, any);
+                    if (bal) {
+                        unsigned long long base = 0;
+                        if (lane == 0) base = atomicAdd(&st->n_cand, (unsigned long long)__popc(bal));
+                        base = __shfl_sync(0xffffffffu, base, 0);
+                        if (any) cand[base + __popc(bal & ((1u << lane) - 1u))] = k;
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
             if (rc[j]) atomicAdd(&h[j][rd[j]], rc[j]);
-            rd[j] = d;
-            rc[j] = 1u;
+        __syncthreads();
+        if (!alone) {
+            for (int j = 0; j < 4; ++j)
+                if (grp[j] == j)
+                    for (int i = threadIdx.x; i < kBins; i += kHistThreads) {
+                        const unsigned int c = h[j][i];
+                        if (c) atomicAdd(hist + j * kBins + i, c);
+                    }
+            __threadfence();
+            __syncthreads();
+            if (threadIdx.x == 0) s_last = atomicAdd(&st->sel_arrive, 1u) == active - 1u;
+            __syncthreads();
+            if (!s_last) return;
+            __threadfence();
+            for (int j = 0; j < 4; ++j)
+                if (grp[j] == j) {
+                    unsigned int c[kBins / kHistThreads];
+#pragma unroll
+                    for (int q = 0; q < kBins / kHistThreads; ++q)
+                        c[q] = __ldcg(hist + j * kBins + threadIdx.x + q * kHistThreads);
+#pragma unroll
+                    for (int q = 0; q < kBins / kHistThreads; ++q) {
+                        h[j][threadIdx.x + q * kHistThreads] = c[q];
+                        hist[j * kBins + threadIdx.x + q * kHistThreads] = 0u;
+                    }
+                }
+            __syncthreads();
         }
-        if (mode == 1) {
-            const unsigned int bal = __ballot_sync(0xffffffffu, any);
-            if (bal) {
-                unsigned long long base = 0;
-                if (lane == 0) base = atomicAdd(&st->n_cand, (unsigned long long)__popc(bal));
-                base = __shfl_sync(0xffffffffu, base, 0);
-                if (any) cand[base + __popc(bal & ((1u << lane) - 1u))] = k;
+        // warp j: target j's digit, the bin whose running total passes its remaining rank.  Lanes
+        // sum 64 bins each (rotated, so that they touch different banks), then the warp scans the
+        // 64 bins of the lane that holds the rank.
+        if (warp < 4) {
+            const unsigned int* hj = h[grp[warp]];
+            constexpr int per = kBins / 32;
+            static_assert(per == 64, "two bins per lane below");
+            unsigned long long inc = 0;
+            for (int q = 0; q < per; ++q) inc += hj[lane * per + ((q + lane) & (per - 1))];
+            const unsigned long long own = inc;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += t;
+            }
+            const unsigned long long rem = __ldcg(&st->rem[warp]);
+            const unsigned int hit = __ballot_sync(0xffffffffu, inc > rem);
+            const int seg = hit ? __ffs(hit) - 1 : 31;
+            const unsigned long long before = __shfl_sync(0xffffffffu, inc - own, seg);
+            const unsigned int c0 = hj[seg * per + 2 * lane], c1 = hj[seg * per + 2 * lane + 1];
+            unsigned long long run = (unsigned long long)c0 + c1;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long t = __shfl_up_sync(0xffffffffu, run, o);
+                if (lane >= o) run += t;
+            }
+            run += before;
+            const unsigned int in = __ballot_sync(0xffffffffu, run > rem);
+            const int at = in ? __ffs(in) - 1 : 31;
+            if (lane == at) {
+                const unsigned long long lo = run - c1 - c0;         // keys below this lane's bins
+                const bool second = lo + c0 <= rem;
+                st->rem[warp] = rem - (second ? lo + c0 : lo);
+                st->prefix[warp] |= (unsigned long long)(seg * per + 2 * lane + (second ? 1 : 0)) << shift;
             }
         }
-      }
+        if (threadIdx.x == 0) {
+            st->sel_arrive = 0u;
+            if (alone && p == kSelPasses - 1) st->sel_done = 1;
+        }
+        __threadfence();
+        __syncthreads();                     // the next pass reads prefix and rem, and clears h
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-        if (rc[j]) atomicAdd(&h[j][rd[j]], rc[j]);
-    __syncthreads();
-    for (int j = 0; j < 4; ++j)
-        if (grp[j] == j)
-            for (int i = threadIdx.x; i < kBins; i += kHistThreads) {
-                const unsigned int c = h[j][i];
-                if (c) atomicAdd(hist + j * kBins + i, c);
-            }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&st->sel_arrive, 1u) == active - 1u;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    for (int j = 0; j < 4; ++j)
-        if (grp[j] == j) {
-            unsigned int c[kBins / kHistThreads];
-#pragma unroll
-            for (int q = 0; q < kBins / kHistThreads; ++q)
-                c[q] = __ldcg(hist + j * kBins + threadIdx.x + q * kHistThreads);
-#pragma unroll
-            for (int q = 0; q < kBins / kHistThreads; ++q) {
-                h[j][threadIdx.x + q * kHistThreads] = c[q];
-                hist[j * kBins + threadIdx.x + q * kHistThreads] = 0u;
-            }
-        }
-    __syncthreads();
-    const int j = threadIdx.x >> 5;
-    if (j < 4) {
-        const unsigned int* hj = h[grp[j]];
-        constexpr int per = kBins / 32;
-        unsigned long long loc = 0;
-        for (int q = 0; q < per; ++q) loc += hj[lane * per + q];
-        unsigned long long inc = loc;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += t;
-        }
-        const unsigned long long rem = st->rem[j];
-        const unsigned int hit = __ballot_sync(0xffffffffu, inc > rem);
-        const int srcl = hit ? __ffs(hit) - 1 : 31;
-        if (lane == srcl) {
-            unsigned long long before = inc - loc;
-            int dsel = lane * per + per - 1;
-            for (int q = 0; q < per; ++q) {
-                const unsigned int c = hj[lane * per + q];
-                if (before + c > rem) { dsel = lane * per + q; break; }
-                before += c;
-            }
-            st->rem[j] = rem - before;
-            st->prefix[j] |= (unsigned long long)dsel << shift;
-        }
-    }
-    if (threadIdx.x == 0) st->sel_arrive = 0u;
 }
 
 // NumPy's _lerp between the order statistics; statistics out.
@@ -641,18 +736,14 @@ int launch_gamma(const GammaParams& P, const T* ref, const T* ev, double* gmap,
         PBD_LAUNCH_CHECK();
         ++launches;
     }
-    const size_t smem = (size_t)(kTX + 2 * P.hx) * (kTY + 2 * P.hy) * (kTZ + 2 * P.hz) *
-                            sizeof(double) +
-                        (size_t)P.n_off * (sizeof(double) + sizeof(int));
+    const size_t smem = gamma_offset_doubles<T>(P.n_off) * sizeof(double) +
+                        (size_t)(kTX + 2 * P.hx) * (kTY + 2 * P.hy) * (kTZ + 2 * P.hz) * sizeof(T);
     int set = 0;                                // once per (device, kernel)
     PBD_TRY(smem_optin((const void*)gamma_kernel<T, false>, kGMaxSmem, 0, &set));
     PBD_TRY(smem_optin((const void*)gamma_kernel<T, true>, kGMaxSmem, 0, &set));
     const int gx = (P.nx + kTX - 1) / kTX, gy = (P.ny + kTY - 1) / kTY;
     const int n_bricks = w.n_blocks;
-    int occ = 0;
-    PBD_TRY(cuda_rc(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, gamma_kernel<T, false>,
-                                                                  kGThreads, smem)));
-    const int grid0 = std::max(1, std::min(n_bricks, std::max(occ, 1) * num_sms()));
+    const int grid0 = n_bricks;      // one block per brick: the masked bricks cost far more than the others
     const int grid1 = std::max(1, std::min(n_bricks, num_sms()));   // fallback: usually idle
     gamma_kernel<T, false><<<grid0, kGThreads, smem, s>>>(P, ref, ev, gmap, mmap, w.st, w.keys,
                                                           w.psum, w.pmax, gx, gy, n_bricks);
@@ -664,11 +755,8 @@ int launch_gamma(const GammaParams& P, const T* ref, const T* ev, double* gmap,
     PBD_LAUNCH_CHECK();
     const int hblocks = num_sms() * 2;
     for (int p = 0; p < kSelPasses; ++p) {
-        const int top = 64 - kDigitBits * p;                       // 64, 53, 42, 31, 20, 9
-        const int shift = top > kDigitBits ? top - kDigitBits : 0;
         const int mode = p < 2 ? 0 : (p == 2 ? 1 : 2);
-        gamma_select_kernel<<<hblocks, kHistThreads, 0, s>>>(w.st, w.keys, w.cand, shift, top,
-                                                             mode, w.hist);
+        gamma_select_kernel<<<hblocks, kHistThreads, 0, s>>>(w.st, w.keys, w.cand, p, mode, w.hist);
         PBD_LAUNCH_CHECK();
     }
     gamma_final_kernel<<<1, 1, 0, s>>>(P, w.st, out, n_offsets);
