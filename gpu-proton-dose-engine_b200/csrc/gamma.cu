@@ -49,7 +49,8 @@ constexpr int kBins = 1 << kDigitBits;
 constexpr int kSelPasses = 6;          // 6 x 11 bits cover the 64-bit keys
 constexpr int kHistThreads = 512;
 constexpr int kFinThreads = 1024;
-constexpr int kSelPer = 16;            // keys per thread a select pass aims at
+constexpr int kSelPer = 4;             // keys per thread a select pass aims at
+constexpr int kSelAlone = 16;          // keys per thread of a block that finishes the candidates alone
 constexpr int kRowBatch = 4;           // staged rows per warp whose loads are issued together
 // largest staged brick (radius 6 on every axis) and offset list (13^3 offsets)
 constexpr int kGMaxOff = 13 * 13 * 13;
@@ -111,6 +112,13 @@ __device__ __forceinline__ double nmin(double a, double b) {
 template <class T>
 __device__ __forceinline__ double ld(const T* p, size_t i) { return (double)__ldg(p + i); }
 
+// The passes after the gamma kernel are short: each is a programmatic dependent of the one before, so
+// that its launch overlaps it; it touches memory only after that grid has completed.
+__device__ __forceinline__ void dependent_start() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 template <class T>
 __global__ void __launch_bounds__(kGThreads)
 gamma_refmax_kernel(const T* __restrict__ ref, size_t n, GammaState* st) {
@@ -125,7 +133,14 @@ gamma_refmax_kernel(const T* __restrict__ ref, size_t n, GammaState* st) {
     for (; i < n; i += stride) best = max(best, dkey(ld(ref, i)));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
-    if ((threadIdx.x & 31) == 0 && best) atomicMax(&st->ref_key, best);
+    // one atomic per block (one per warp, all on one address, were most of the kernel's time)
+    __shared__ unsigned long long red[kGThreads / 32];
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = best;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kGThreads / 32; ++w) best = max(best, red[w]);
+        if (best) atomicMax(&st->ref_key, best);
+    }
 }
 
 // Doses and criteria inside [1 / kTame, kTame] in magnitude go through the screen: nothing overflows
@@ -384,6 +399,7 @@ __global__ void __launch_bounds__(kFinThreads)
 gamma_finish_kernel(const GammaParams P, GammaState* st, const double* __restrict__ part_sum,
                     const double* __restrict__ part_max, int grid0, int grid1) {
     __shared__ double s_sum[kFinThreads / 32], s_max[kFinThreads / 32];
+    dependent_start();
     if (st->status != 0) return;
     const int pass = st->cnt[0][0] != 0ull ? 0 : 1;
     const int n_blocks = pass ? grid1 : grid0;
@@ -440,22 +456,24 @@ gamma_finish_kernel(const GammaParams P, GammaState* st, const double* __restric
 // candidate list; mode 2 reads only the candidates.  The grid is trimmed to about kSelPer keys per
 // thread; once one block is enough for the candidates (nearly always), it takes all the passes that
 // are left without the global histogram, and the launches after it have nothing to do.
-// 128^3: six passes of 11 us with a bin scan that conflicted on one bank, together
-// 57 us now.
+// Bound by latency: reading the state, the keys, the global histogram's atomics and the last block's
+// scan follow one another, 8-14 us a pass.  From the finish kernel to the interpolation (128^3, 434,000
+// masked voxels): 85 us as plain launches with 16 keys per thread and a bin scan on one bank, now 60.
 __global__ void __launch_bounds__(kHistThreads)
 gamma_select_kernel(GammaState* st, const unsigned long long* __restrict__ keys,
                     unsigned long long* __restrict__ cand, int pass, int mode,
                     unsigned int* __restrict__ hist) {
     __shared__ unsigned int h[4][kBins];
     __shared__ int s_last;
+    dependent_start();
     if (st->status != 0 || st->sel_done) return;
     const unsigned long long n = mode == 2 ? st->n_cand : st->n_eval;
     const unsigned long long* src = mode == 2 ? cand : keys;
     const unsigned long long want = (n + (unsigned long long)kHistThreads * kSelPer - 1) /
                                     ((unsigned long long)kHistThreads * kSelPer);
-    const unsigned int active = (unsigned int)(want < gridDim.x ? (want ? want : 1) : gridDim.x);
+    const bool alone = mode == 2 && n <= (unsigned long long)kHistThreads * kSelAlone;
+    const unsigned int active = alone ? 1u : (unsigned int)(want < gridDim.x ? (want ? want : 1) : gridDim.x);
     if (blockIdx.x >= active) return;
-    const bool alone = mode == 2 && active == 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int p = pass; p < (alone ? kSelPasses : pass + 1); ++p) {
         const int top = 64 - kDigitBits * p;                       // 64, 53, 42, 31, 20, 9
@@ -495,6 +513,12 @@ gamma_select_kernel(GammaState* st, const unsigned long long* __restrict__ keys,
                 const unsigned long long k = kk[q];
                 const unsigned int d = (unsigned int)(k >> shift) & dmask;
                 bool any = false;
+                if (p == 0) {
+                    // one prefix, few digits (sign and exponent): one atomic per digit and warp
+                    const unsigned same = __match_any_sync(0xffffffffu, valid ? d : ~0u);
+                    if (valid && lane == __ffs(same) - 1) atomicAdd(&h[0][d], (unsigned)__popc(same));
+                    continue;
+                }
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     if (grp[j] != j || !valid || (k & himask) != pre[j]) continue;
@@ -594,6 +618,7 @@ gamma_select_kernel(GammaState* st, const unsigned long long* __restrict__ keys,
 // NumPy's _lerp between the order statistics; statistics out.
 __global__ void gamma_final_kernel(const GammaParams P, GammaState* st, pbd_gamma_stats* out,
                                    int n_offsets) {
+    dependent_start();
     pbd_gamma_stats r;
     memset(&r, 0, sizeof(r));
     r.status = st->status;
@@ -726,8 +751,8 @@ int launch_gamma(const GammaParams& P, const T* ref, const T* ev, double* gmap,
                  unsigned char* mmap, const GammaWs& w, pbd_gamma_stats* out, int n_offsets,
                  cudaStream_t s) {
     const size_t n = (size_t)P.nz * P.ny * P.nx;
-    PBD_TRY(cuda_rc(cudaMemsetAsync(w.st, 0, sizeof(GammaState), s)));
-    PBD_TRY(cuda_rc(cudaMemsetAsync(w.hist, 0, 4 * kBins * sizeof(unsigned int), s)));
+    // the state and the histogram behind it
+    PBD_TRY(cuda_rc(cudaMemsetAsync(w.st, 0, (char*)(w.hist + 4 * kBins) - (char*)w.st, s)));
     int launches = 0;
     if (!P.use_ref_dose) {
         const int blocks = (int)std::min<size_t>((n + kGThreads - 1) / kGThreads,
@@ -751,16 +776,15 @@ int launch_gamma(const GammaParams& P, const T* ref, const T* ev, double* gmap,
     gamma_kernel<T, true><<<grid1, kGThreads, smem, s>>>(P, ref, ev, gmap, mmap, w.st, w.keys,
                                                          w.psum, w.pmax, gx, gy, n_bricks);
     PBD_LAUNCH_CHECK();
-    gamma_finish_kernel<<<1, kFinThreads, 0, s>>>(P, w.st, w.psum, w.pmax, grid0, grid1);
-    PBD_LAUNCH_CHECK();
+    PBD_TRY(launch_dependent(gamma_finish_kernel, dim3(1), dim3(kFinThreads), 0, s, P, w.st,
+                             (const double*)w.psum, (const double*)w.pmax, grid0, grid1));
     const int hblocks = num_sms() * 2;
     for (int p = 0; p < kSelPasses; ++p) {
         const int mode = p < 2 ? 0 : (p == 2 ? 1 : 2);
-        gamma_select_kernel<<<hblocks, kHistThreads, 0, s>>>(w.st, w.keys, w.cand, p, mode, w.hist);
-        PBD_LAUNCH_CHECK();
+        PBD_TRY(launch_dependent(gamma_select_kernel, dim3(hblocks), dim3(kHistThreads), 0, s, w.st,
+                                 (const unsigned long long*)w.keys, w.cand, p, mode, w.hist));
     }
-    gamma_final_kernel<<<1, 1, 0, s>>>(P, w.st, out, n_offsets);
-    PBD_LAUNCH_CHECK();
+    PBD_TRY(launch_dependent(gamma_final_kernel, dim3(1), dim3(1), 0, s, P, w.st, out, n_offsets));
     count_launch(launches + 4 + kSelPasses);
     return PBD_OK;
 }
