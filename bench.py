@@ -971,7 +971,7 @@ def main():
     # the split forms' own ceiling: TF32 runs at half the BF16 rate, three products per MAC
     # (BF16x3: the BF16 rate, three products); credited FLOPs count one product
     split_ceiling = {"fp16x3": peak / 3.0, "tf32x3": peak / 6.0, "bf16x3": peak / 3.0,
-                     "tf32": peak / 2.0, "bf16": peak}.get(prec if dom == "forward" else "bf16x3")
+                     "tf32": peak / 2.0, "bf16": peak}.get(prec if dom == "forward" else "fp16x3")
     roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak, "traffic": read_traffic(kname), "kernel": kname,
             "kernel_ms_per_launch": dom_ms, "flop_per_launch": per_launch_flop,
@@ -984,7 +984,7 @@ def main():
             "fwd_ms_per_launch": prof["fwd_ms"] / max(prof["n_fwd"], 1),
             "adj_ms_per_launch": prof["adj_ms"] / max(prof["n_adj"], 1)}
 
-    adj_mode = {"fp16x3": "bf16x3", "tf32x3": "bf16x3", "tf32": "bf16x3", "bf16x3": "bf16x3",
+    adj_mode = {"fp16x3": "fp16x3", "tf32x3": "fp16x3", "tf32": "fp16x3", "bf16x3": "fp16x3",
                 "bf16": "bf16", "fp32": "fp32"}[prec]
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": K,
             "warmup": max(args.warmup, 3), "ms_per_step": t_ms / K, "higher_is_better": True,

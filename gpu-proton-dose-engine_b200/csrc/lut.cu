@@ -590,7 +590,7 @@ lut_eval_kernel(pbd_lut_spec spec, LutDims dm, const LayerScal* __restrict__ sca
 
 // Heterogeneous media: dose = sum_l IDD_l(WED) * lateral_l per voxel, IDD_l the layer's
 // smoothed depth curve evaluated at the voxel's water-equivalent depth with the same
-// interpolation as the tables (lut_output_kernel).  Accumulated in FP64, in layer order.
+// interpolation as the tables.  Accumulated in FP64, in layer order.
 //
 // A warp owns 128 consecutive voxels (4 per lane, lanes adjacent) and walks the layers that reach any
 // of them, the next layer's lateral values loaded while this one's curve points are gathered; layers

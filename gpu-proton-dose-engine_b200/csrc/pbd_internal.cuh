@@ -223,8 +223,8 @@ int launch_forward_tc(int precision, JobDev* jobs_dev, const JobDev* jobs_host, 
                       int* counter, int* err, int chunk, int with_loss, int poison,
                       cudaStream_t s);
 
-// forward in FP64 on the CUDA cores -- fwd_f64.cu.  One block per (slice, 64 x 64 tile)
-// over all layers, writing the dose directly (no scratch).
+// forward in FP64 (mma.sync f64) -- fwd_f64.cu.  One block per (slice, tile) over all layers,
+// writing the dose directly (no scratch).
 int launch_forward_f64(const pbd_field* f, const double* w, const double* idd,
                        const double* sigma, double* dose, cudaStream_t s);
 

@@ -54,12 +54,14 @@ extern "C" {
 
 /* Arithmetic used for the two Gaussian contractions.  All accumulate in FP32. */
 #define PBD_PREC_FP32    0   /* FP32 FMA on the CUDA cores */
-#define PBD_PREC_TF32X3  1   /* tcgen05 TF32, hi/lo split, three products */
+#define PBD_PREC_TF32X3  1   /* tcgen05 TF32, hi/lo split, three products (the lateral maps of a
+                                dose in a medium: as FP16X3, which is nearer to 64 bits) */
 #define PBD_PREC_TF32    2   /* tcgen05 TF32, one product */
 #define PBD_PREC_BF16X3  3   /* tcgen05 BF16, hi/lo split, three products */
 #define PBD_PREC_BF16    4   /* tcgen05 BF16, one product */
 #define PBD_PREC_FP16X3  5   /* tcgen05 FP16, hi/lo split, three products; operands scaled by
-                                powers of two into FP16's range */
+                                powers of two into FP16's range.  The adjoint of every mode but
+                                FP32 and BF16 */
 
 #define PBD_MAX_JOBS 128     /* jobs (fields x scenarios) per batched launch */
 
