@@ -150,43 +150,6 @@ __device__ __forceinline__ void locate_lin(double x, double a, double b, int n, 
     x0_out = x0;
 }
 
-// locate_lin on linspace(0, zmax, n) for 0 <= x <= zmax (or NaN: some lo in range): the estimate
-// floor(x inv) by adding 1.5 2^52, whose sum's low word is the integer -- two FP64 additions
-// instead of two conversions at a quarter of their rate -- then the same correction.
-__device__ __forceinline__ void locate_curve(double x, double zmax, int n, double step, double inv,
-                                             int& lo_out, double& x0_out) {
-    constexpr double kMagic = 6755399441055744.0;
-    const double t = (x * inv - 0.5) + kMagic;
-    int lo = __double2loint(t);
-    double fk = t - kMagic;
-    if (lo < 0 || lo > n - 2) {
-        lo = lo < 0 ? 0 : n - 2;
-        fk = (double)lo;
-    }
-    double x0 = fk * step;
-    if (x0 > x && lo > 0) {
-        do {
-            --lo;
-            fk -= 1.0;
-            x0 = fk * step;
-        } while (lo > 0 && x0 > x);
-    } else {
-        while (lo < n - 2) {
-            const double x1 = lo + 1 == n - 1 ? zmax : (fk + 1.0) * step;
-            if (!(x1 <= x)) break;
-            ++lo;
-            fk += 1.0;
-            x0 = x1;
-        }
-    }
-    if (x == zmax) {
-        lo = n - 1;
-        x0 = zmax;
-    }
-    lo_out = lo;
-    x0_out = x0;
-}
-
 __device__ __forceinline__ double csda(double e) {
     return interp(e, g_etab, g_rtab, kTableN, g_rtab[0], g_rtab[kTableN - 1]);
 }
@@ -687,19 +650,25 @@ __global__ void __launch_bounds__(kCmbThreads, 4) wed_combine_kernel(
         if (v0 + 32 * j < nvox) __stcs(dose + v0 + 32 * j, bad ? __int_as_float(0x7fc00000) : (float)acc[j]);
 }
 
-// Depth dose of a layer's curve {value, slope} at depth d (np.interp's interval and value, 0
-// outside [0, zmax]); scalars as in LayerScal.
+// Depth dose of a layer's curve {value, slope} at depth d, 0 outside [0, zmax]: the interval is the
+// rounded estimate alone, as in the combine (any d, NaN included, gives an index inside the curve);
+// scalars as in LayerScal.
 struct CurveScal {
     double zmax, step, inv;
 };
-__device__ __forceinline__ double curve_at(const CurveScal& c, const double2* __restrict__ pts, int n,
-                                           double d) {
-    if (d < 0.0 || d > c.zmax) return 0.0;
-    int lo = 0;
-    double x0 = 0.0;
-    locate_curve(d, c.zmax, n, c.step, c.inv, lo, x0);
-    const double2 pt = __ldg(pts + lo);
-    return x0 == d ? pt.x : pt.y * (d - x0) + pt.x;
+struct CurvePoint {
+    double2 pt;
+    double x;                // from the interval's left point
+};
+__device__ __forceinline__ CurvePoint curve_point(const CurveScal& c, const double2* __restrict__ pts,
+                                                  int n, double d) {
+    constexpr double kMagic = 6755399441055744.0;
+    const double t = fma(d, c.inv, -0.5) + kMagic;
+    const unsigned lo = min((unsigned)__double2loint(t), (unsigned)(n - 1));
+    return CurvePoint{__ldg(pts + lo), fma(kMagic - t, c.step, d)};
+}
+__device__ __forceinline__ double curve_value(const CurvePoint& p, double zmax, double d) {
+    return d < 0.0 || d > zmax ? 0.0 : fma(p.pt.y, p.x, p.pt.x);
 }
 
 // The heterogeneous dose's dL/dD seen by layer l: maps[l * lstride + v] = IDD_l(WED[v]) *
@@ -710,12 +679,11 @@ __device__ __forceinline__ double curve_at(const CurveScal& c, const double2* __
 // one FP32 rounding of the product).  Only slices that the layer's activity table (act, act +
 // act_stride) marks are written: the adjoint reads no other.
 //
-// One block per 512 voxels of a slice, two per thread, over the slice's active layers.  Bound by
-// FP64 issue: some 12 operations per curve, the interval located without integer conversions
-// (a quarter of the FP64 rate).  One pass for both sets reads the WED and dL/dD once, and about
-// half of the (layer, slice) pairs are inactive: 128^3 x 28 layers, both sets, 497 us as two
-// kernels over every pair with a division per curve, 240 us
-// now, half of it the gathers of the curve points through L1.
+// One block per 512 voxels of a slice, two per thread, over the slice's active layers.  Bound by the
+// gathers of the curve points through L1 and their latency: both voxels' points of all three curves
+// are in flight together.  128^3 x 28 layers, both sets: 497 us as two kernels over every pair with
+// a division per curve; 240 us in one pass over the active pairs (about half) with np.interp's exact
+// interval; 150 us now, with the estimated interval and the points loaded ahead.
 constexpr int kMapThreads = 256, kMapPer = 2;
 constexpr int kMapLayers = 128;   // layers staged together
 
@@ -776,19 +744,27 @@ __global__ void __launch_bounds__(kMapThreads) wed_grad_maps_kernel(
         for (int k = 0; k < na; ++k) {
             const unsigned f = (unsigned)s_l[k];
             const size_t l = f & 0x3FFFFFFFu;
+            // every curve point of the layer in flight together, whichever sets are written
+            CurvePoint p[kRange ? 3 : 1][kMapPer];
+#pragma unroll
+            for (int q = 0; q < kMapPer; ++q) {
+                p[0][q] = curve_point(s_c[0][k], pts + l * n, n, d[q]);
+                if constexpr (kRange) {
+                    p[1][q] = curve_point(s_c[1][k], ptp + l * n, n, d[q]);
+                    p[2][q] = curve_point(s_c[2][k], ptm + l * n, n, d[q]);
+                }
+            }
             if (f & (1u << 30)) {
 #pragma unroll
-                for (int q = 0; q < kMapPer; ++q) {
-                    const double idd = curve_at(s_c[0][k], pts + l * n, n, d[q]);
-                    if (in[q]) out[q][l * lstride] = (float)(idd * g[q]);
-                }
+                for (int q = 0; q < kMapPer; ++q)
+                    if (in[q]) out[q][l * lstride] = (float)(curve_value(p[0][q], s_c[0][k].zmax, d[q]) * g[q]);
             }
             if constexpr (kRange) {
                 if (f & (1u << 31)) {
 #pragma unroll
                     for (int q = 0; q < kMapPer; ++q) {
-                        const double dp = curve_at(s_c[1][k], ptp + l * n, n, d[q]);
-                        const double dm = curve_at(s_c[2][k], ptm + l * n, n, d[q]);
+                        const double dp = curve_value(p[1][q], s_c[1][k].zmax, d[q]);
+                        const double dm = curve_value(p[2][q], s_c[2][k].zmax, d[q]);
                         if (in[q]) out[q][set_stride + l * lstride] = (float)((dp - dm) * inv2h * g[q]);
                     }
                 }

@@ -51,6 +51,27 @@ def test_dose_vs_oracle(pb, shape, prec):
     assert np.max(np.abs(got - want)) <= 1e-6 * np.max(np.abs(want))
 
 
+@pytest.mark.parametrize("shape", [(37, 50, 6, 17, 33, 3), (128, 5, 4, 3, 2, 131)])
+def test_gradients_vs_oracle(pb, shape):
+    """dL/dW and dL/dR with water-equivalent depths inside no curve, on the curves' far ends and over 128
+    layers; 1e-5 of the largest (the adjoint's split FP16 is good to some 1e-6)."""
+    import torch
+    prob, en, sig, rho = _problem(pb, *shape, seed=sum(shape))
+    g, L = prob.grid, prob.lattice
+    wed = hr.wed_ref(rho, g.oz, g.dz)
+    wed[0, 0, 0], wed[-1, -1, -1], wed[1, 0, 0] = -0.3, 1e6, 0.0
+    grad = np.random.default_rng(2).standard_normal(wed.shape).astype(np.float32)
+    w = np.float32(L.weights)
+    want = hr.grad_w_ref(g.x, g.y, L.spot_x, L.spot_y, w, en, sig, wed, grad.astype(np.float64))
+    plan = pb.hetero.WedPlan(prob)
+    gw, gr = plan.adjoint(torch.as_tensor(grad, device="cuda"), torch.as_tensor(wed), with_range=True)
+    assert np.max(np.abs(gw.cpu().numpy() - want)) <= 1e-5 * np.max(np.abs(want))
+    assert torch.equal(gw, plan.adjoint(torch.as_tensor(grad, device="cuda"), torch.as_tensor(wed)))
+    zc = g.oz + np.arange(g.nz) * g.dz
+    want_r = hr.grad_range_ref(g.x, g.y, L.spot_x, L.spot_y, w, en, zc, wed, grad.astype(np.float64), plan.fd_step)
+    assert np.max(np.abs(gr.cpu().numpy() - want_r)) <= 1e-4 * np.max(np.abs(want_r))
+
+
 @pytest.mark.parametrize("shape", [(1, 1, 1), (128, 3, 33), (129, 5, 31), (257, 2, 40)])
 @pytest.mark.parametrize("oz", [0.0, -1.3, 2.1])
 def test_raytrace_vs_oracle(pb, shape, oz):
