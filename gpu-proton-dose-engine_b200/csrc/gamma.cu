@@ -503,7 +503,7 @@ gamma_select_kernel(GammaState* st, const unsigned long long* __restrict__ keys,
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const unsigned long long i = b0 + q * stride + lane;
-                kk[q] = i < n ? __ldg(src + i) : 0ull;
+                kk[q] = i < n ? __ldcg(src + i) : 0ull;   // not __ldg: written after this grid was launched
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
