@@ -118,8 +118,12 @@ struct Params {
     int hold;            // test of the timeout path: the scheduler publishes no step
     int N1;              // x-lattice padded to 16
     int tiles;           // 128-row tiles whose G^T the shared memory holds (1 or 2)
-    int stage;           // 1: each unit's dL/dD slice arrives by bulk copy into a staging buffer
-                         //    (one tile; every job's slice is contiguous, 16-byte aligned, nx ny % 4 == 0)
+    int stage;           // each unit's dL/dD slice arrives in a staging buffer: 1 by bulk copy (every job's
+                         //    slice 16-byte aligned, nx ny % 4 == 0), 2 by 4-byte cp.async (any other), 0:
+                         //    read from global memory (several tiles).  Read from global memory as well,
+                         //    a slice of the second kind took 10 us a unit where no other step hid it:
+                         //    5 layers of 53 x 53 x 110 in a medium 76 us against 40, and
+                         //    117 x 93 x 121 with 33 layers' adjoint 93 us against 86
     uint32_t o_b2, o_w, w_bytes, o_stage;   // shared-memory offsets: B, weights (two buffers), staging
     int sym;             // 1: every job is one tile and symmetric in x and y (grid, lattice, origins),
                          //    so B's rows equal the rows G evaluates for A
@@ -268,9 +272,20 @@ __device__ __forceinline__ void scheduler_warp(const Params& P, const Units U, S
             bool w = true;
             if (nu > 0) w = wait_bar(B.sfree, (uint32_t)((nu - 1) & 1), P.wait_ns);
             if (!__all_sync(FULL, w)) { ok = false; break; }
-            if (lane == 0) {
+            const uint32_t dst = tc::smem_u32(smem) + P.o_stage;
+            if (P.stage == 2) {
+                // a slice without 16-byte alignment: coalesced 4-byte copies by all lanes, each of
+                // which arrives when its own have landed
+                const float* src = J.grad_dose + (size_t)z * J.ny * J.nx;
+                const int n = J.nx * J.ny;
+#pragma unroll 8
+                for (int e = lane; e < n; e += 32)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4u * (uint32_t)e), "l"(src + e)
+                                 : "memory");
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc::smem_u32(B.sfull))
+                             : "memory");
+            } else if (lane == 0) {
                 const uint32_t bytes = (uint32_t)J.nx * (uint32_t)J.ny * 4u;
-                const uint32_t dst = tc::smem_u32(smem) + P.o_stage;
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
                                  tc::smem_u32(B.sfull)), "r"(bytes)
                              : "memory");
@@ -647,8 +662,8 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
         if (cur.flags & kFirst) {
             const JobDev& J = P.jobs[cur.job];
             const int nx = J.nx, ny = J.ny, x0 = cur.xt * kTile;
-            // the slice from the staging buffer (bulk copy issued by the scheduler when it
-            // claimed the unit) or, for slices that cannot be bulk copied, from global memory
+            // the slice from the staging buffer (copied by the scheduler when it claimed the unit) or,
+            // with several tiles, from global memory
             const float* g = J.grad_dose + (size_t)cur.z * ny * nx + x0;
             if (P.stage) {
                 ok = wait_bar(B.sfull, (uint32_t)(nu & 1), P.wait_ns);
@@ -665,6 +680,8 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
                     const uint4 a = sv[e];
                     mx = max(max(mx, a.x & 0x7FFFFFFFu), max(a.y & 0x7FFFFFFFu, max(a.z & 0x7FFFFFFFu, a.w & 0x7FFFFFFFu)));
                 }
+                if (tid < (nx * ny & 3))
+                    mx = max(mx, reinterpret_cast<const unsigned*>(sv)[(nx * ny & ~3) + tid] & 0x7FFFFFFFu);
             } else {
                 const int xw = min(kTile, nx - x0);
 #pragma unroll 16
@@ -917,7 +934,7 @@ __global__ void __launch_bounds__(kThreads, 1) adj_tc_kernel(Params P) {
             tc::mbar_init(&B.full[i], 1);
             tc::mbar_init(&B.empty[i], kMathWarps + 3);   // math warps, both MMA warps, weight warp
         }
-        tc::mbar_init(B.sfull, 1);                        // the scheduler's expect_tx + bytes
+        tc::mbar_init(B.sfull, P.stage == 2 ? 32 : 1);     // the scheduler's lanes, or its expect_tx + bytes
         tc::mbar_init(B.sfree, kMathWarps);
         tc::mbar_init(B.ops1, kMathWarps);
         tc::mbar_init(B.ops2, kMathWarps);
@@ -1204,7 +1221,7 @@ int launch_adjoint_tc(int precision, JobDev* jobs_dev, const JobDev* jobs_host, 
         PBD_TRY(tc_adjoint_dims_tiled(precision, &f, &n1));
         if (((size_t)J.nx * J.ny) % 4 != 0 ||
             (reinterpret_cast<uintptr_t>(J.grad_dose) & 15u) != 0)
-            P.stage = 0;
+            P.stage = 2;
         P.N1 = std::max(P.N1, n1);
         P.tiles = std::max(P.tiles, J.nty);
         P.xtmax = std::max(P.xtmax, J.ntx);
