@@ -22,16 +22,24 @@ namespace {
 
 constexpr int NT = 256;
 constexpr int SC = kSpotChunk;                      // 64 spots per chunk
-// shared memory of a 16 RY x 16 RX tile with spot chunks of sc (128 x 128, 64 spots: 112 KiB)
-constexpr size_t fwd_smem(int ry, int rx, int sc) {
-    return (size_t)(sc * 16 * (2 * rx + ry) + sc * SC) * sizeof(float);
+// shared memory of a 16 RY x 16 RX tile with spot chunks of scx x scy (128 x 128, 64 x 64 spots: 112 KiB)
+constexpr size_t fwd_smem(int ry, int rx, int scx, int scy) {
+    return (size_t)(16 * (rx * scx + (rx + ry) * scy) + scx * SC) * sizeof(float);
+}
+// Spots per chunk of an axis of n: equal parts of at most 64, in fours (73 spots as 40 + 33, not 64 + 9).
+// Each axis of each job has its own.  One size for the launch, from its widest axis, cut 41 spots beside
+// 73 into 40 + 1, each part with its own weights, factors and barriers: 128 x 128 x 64, 73 x 41 spots,
+// 10 layers 302 us, now 217; a batch of three 41 x 41 fields and a small one of 73 x 73 386, now 306.
+__host__ __device__ constexpr int spot_chunk(int n) {
+    const int parts = (n + SC - 1) / SC;
+    return ((n + parts - 1) / parts + 3) / 4 * 4;
 }
 
 // Tile sizes per axis, in units of 16 voxels.  An axis of n voxels is cut into ceil(n / 128) tiles of
 // equal size, rounded up to one of these: a 150 x 142 slice in four 80 x 80 tiles instead of four
 // 128 x 128 ones, of which two thirds were outside the grid.  The kernel is bound by FP32 FMA issue, so
-// its time follows the padded area: 150 x 142 x 160, 24 layers of 73 x 73 spots (cut in chunks of 37 for
-// the same reason, where 64 + 9 were padded to 128): 1143 us with 128 x 128 tiles and 64-spot chunks, 640
+// its time follows the padded area: 150 x 142 x 130, 24 layers of 73 x 69 spots (cut in chunks of 40 and 36
+// for the same reason, where 64 + 9 were padded to 128): 1143 us with 128 x 128 tiles and 64-spot chunks, 640
 // with these, 605-626 with three blocks to an SM (which small tiles allow and large ones do not: an
 // 8 x 8 register tile needs 128 registers).  A grid of 128 keeps its 128 x 128 tile: two of 64 x 128
 // would build every factor of the uncut axis twice.  Sums run in the same order whatever the tile.
@@ -162,14 +170,14 @@ __device__ __forceinline__ void stage1(const float* WT, const float* GxT, int ni
 template <int RY, int RX>
 __global__ void __launch_bounds__(NT, RY * RX <= 25 ? 3 : 2)
 fwd_simt_kernel(const JobDev* __restrict__ jobs, const FwdItem* __restrict__ items, int total,
-                int* counter, int sc) {
+                int* counter, int mx, int my) {
     constexpr int TY = 16 * RY, TX = 16 * RX;
     constexpr int PX = NT / TX, PY = NT / TY;        // spots generated at a time
     extern __shared__ float4 smem4[];
-    float* GxT = reinterpret_cast<float*>(smem4);   // [sc i][TX x]
-    float* GyT = GxT + sc * TX;                      // [sc j][TY y]
-    float* U = GyT + sc * TY;                        // [sc j][TX x]
-    float* WT = U + sc * TX;                         // [sc i][SC j]
+    float* GxT = reinterpret_cast<float*>(smem4);   // [mx i][TX x], mx x my: the largest chunk of any job
+    float* GyT = GxT + mx * TX;                      // [my j][TY y]
+    float* U = GyT + my * TY;                        // [my j][TX x]
+    float* WT = U + my * TX;                         // [mx i][SC j]
     __shared__ int s_item;
     __shared__ double s_xs[SC], s_ys[SC];
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
@@ -186,6 +194,7 @@ fwd_simt_kernel(const JobDev* __restrict__ jobs, const FwdItem* __restrict__ ite
         const JobDev& J = jobs[it.job];
         const int nz = J.nz, nx = J.nx, ny = J.ny, nsx = J.nsx, nsy = J.nsy;
         const int z = it.z, y0 = it.ty * TY, x0 = it.tx * TX;
+        const int scx = spot_chunk(nsx), scy = spot_chunk(nsy);
         const double cx = 0.5 * (double)(nsx - 1), cy = 0.5 * (double)(nsy - 1);
         const double xv = J.ox + (double)(x0 + gx) * J.dx, yv = J.oy + (double)(y0 + gy) * J.dy;
 
@@ -203,16 +212,16 @@ fwd_simt_kernel(const JobDev* __restrict__ jobs, const FwdItem* __restrict__ ite
             const float nrm = (float)(c * kInv2Pi / (s * s));
             const float* wl = J.w + (size_t)l * nsy * nsx;
 
-            for (int j0 = 0; j0 < nsy; j0 += sc) {
-                const int nj = min(sc, nsy - j0);
+            for (int j0 = 0; j0 < nsy; j0 += scy) {
+                const int nj = min(scy, nsy - j0);
                 float uacc[4][RX];
 #pragma unroll
                 for (int a = 0; a < 4; ++a)
 #pragma unroll
                     for (int b = 0; b < RX; ++b) uacc[a][b] = 0.f;
 
-                for (int i0 = 0; i0 < nsx; i0 += sc) {
-                    const int ni = min(sc, nsx - i0);
+                for (int i0 = 0; i0 < nsx; i0 += scx) {
+                    const int ni = min(scx, nsx - i0);
                     __syncthreads();
                     // a thread forms the factors of one column (row) of the tile, every PX-th (PY-th)
                     // spot: its voxel's position stays in a register
@@ -316,7 +325,7 @@ __global__ void fwd_finalize_kernel(const JobDev* __restrict__ jobs, int with_lo
     }
 }
 
-using FwdKernel = void (*)(const JobDev*, const FwdItem*, int, int*, int);
+using FwdKernel = void (*)(const JobDev*, const FwdItem*, int, int*, int, int);
 template <int RY>
 FwdKernel pick_rx(int rx) {
     switch (rx) {
@@ -390,20 +399,23 @@ int launch_forward(JobDev* jobs_dev, const JobDev* jobs_host, int n_jobs, FwdIte
         ry = std::max(ry, tile_size(jobs_host[j].ny));
         rx = std::max(rx, tile_size(jobs_host[j].nx));
     }
-    // spot chunks: the widest lattice in equal parts of at most 64 (73 spots as 37 + 36, not 64 + 9)
-    int ns = 1;
-    for (int j = 0; j < n_jobs; ++j) ns = std::max(ns, std::max(jobs_host[j].nsx, jobs_host[j].nsy));
-    const int parts = (ns + SC - 1) / SC, sc = ((ns + parts - 1) / parts + 3) / 4 * 4;
+    // the largest spot chunks of any job size the shared memory
+    int mx = 4, my = 4;
+    for (int j = 0; j < n_jobs; ++j) {
+        mx = std::max(mx, spot_chunk(jobs_host[j].nsx));
+        my = std::max(my, spot_chunk(jobs_host[j].nsy));
+    }
     const FwdKernel kernel = pick_kernel(ry, rx);
-    PBD_TRY(smem_optin((const void*)kernel, (int)fwd_smem(ry, rx, SC), 0, &set));
+    PBD_TRY(smem_optin((const void*)kernel, (int)fwd_smem(ry, rx, SC, SC), 0, &set));
     PBD_TRY(cuda_rc(cudaMemsetAsync(counter, 0, sizeof(int), s)));
     fwd_schedule_kernel<<<n_jobs, 256, kActStage, s>>>(jobs_dev, items, chunk);
     PBD_LAUNCH_CHECK();
     {
-        const int per_sm = ry * rx <= 25 && 3 * (fwd_smem(ry, rx, sc) + 2048u) <= 228u * 1024u ? 3 : 2;
+        const size_t smem = fwd_smem(ry, rx, mx, my);
+        const int per_sm = ry * rx <= 25 && 3 * (smem + 2048u) <= 228u * 1024u ? 3 : 2;
         const int grid = max(1, min(total_items, per_sm * num_sms()));
         prof_mark(kProfFwd, 0, s);
-        kernel<<<grid, NT, fwd_smem(ry, rx, sc), s>>>(jobs_dev, items, total_items, counter, sc);
+        kernel<<<grid, NT, smem, s>>>(jobs_dev, items, total_items, counter, mx, my);
         PBD_LAUNCH_CHECK();
         prof_mark(kProfFwd, 1, s);
     }
