@@ -81,3 +81,10 @@ def test_uneven_lattice_has_a_chunk_per_axis(pb):
     p40, p41 = (_problem(pb, 128, 128, 64, 73, n, 10) for n in (40, 41))
     t40, t41 = _times(_batch(pb, [p40]), _batch(pb, [p41]))
     assert t41 <= 1.2 * t40              # 1.39 times with one chunk size for both axes, 1.02 with one each
+
+
+def test_more_than_60_spots_run_two_blocks_to_an_sm(pb):
+    """Chunks of 64 spots take the most shared memory: 61 spots take about as long as 60."""
+    p60, p61 = (_problem(pb, 200, 200, 64, n, n, 10) for n in (60, 61))
+    t60, t61 = _times(_batch(pb, [p60]), _batch(pb, [p61]))
+    assert t61 <= 1.12 * t60             # 1.26 times with one block to an SM, 1.01 with two
