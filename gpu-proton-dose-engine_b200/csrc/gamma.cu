@@ -52,10 +52,20 @@ constexpr int kFinThreads = 1024;
 constexpr int kSelPer = 4;             // keys per thread a select pass aims at
 constexpr int kSelAlone = 16;          // keys per thread of a block that finishes the candidates alone
 constexpr int kRowBatch = 4;           // staged rows per warp whose loads are issued together
-// largest staged brick (radius 6 on every axis) and offset list (13^3 offsets)
+// Doubles that the gamma kernel's offset tables (weights in FP64 and in T, positions) take before the tile,
+// and bytes of its shared memory for n_off offsets and radii hx, hy, hz.
+template <class T>
+constexpr __host__ __device__ size_t gamma_offset_doubles(int n_off) {
+    return ((size_t)n_off * (sizeof(double) + sizeof(T) + sizeof(int)) + 7) / 8;
+}
+template <class T>
+constexpr size_t gamma_smem(int n_off, int hx, int hy, int hz) {
+    return gamma_offset_doubles<T>(n_off) * sizeof(double) +
+           (size_t)(kTX + 2 * hx) * (kTY + 2 * hy) * (kTZ + 2 * hz) * sizeof(T);
+}
+// the largest: radius 6 on every axis, 13^3 offsets
 constexpr int kGMaxOff = 13 * 13 * 13;
-constexpr int kGMaxSmem = (kTX + 12) * (kTY + 12) * (kTZ + 12) * (int)sizeof(double) +
-                          kGMaxOff * (int)(2 * sizeof(double) + sizeof(int));
+constexpr int kGMaxSmem = (int)gamma_smem<double>(kGMaxOff, 6, 6, 6);
 
 struct GammaParams {
     int nz, ny, nx;
@@ -155,12 +165,6 @@ template <> struct Screen<double> { static constexpr double rel = 0x1p-46; };
 
 __device__ __forceinline__ double local_crit(const GammaParams& P, double r, double crit_g) {
     return P.local ? __dmul_rn(P.crit_frac, r > 1e-12 || r != r ? r : 1e-12) : crit_g;
-}
-
-// Doubles that the offset tables (weights in FP64 and in T, positions) take before the tile.
-template <class T>
-constexpr __host__ __device__ size_t gamma_offset_doubles(int n_off) {
-    return ((size_t)n_off * (sizeof(double) + sizeof(T) + sizeof(int)) + 7) / 8;
 }
 
 template <class T, bool kFallback>
@@ -761,8 +765,7 @@ int launch_gamma(const GammaParams& P, const T* ref, const T* ev, double* gmap,
         PBD_LAUNCH_CHECK();
         ++launches;
     }
-    const size_t smem = gamma_offset_doubles<T>(P.n_off) * sizeof(double) +
-                        (size_t)(kTX + 2 * P.hx) * (kTY + 2 * P.hy) * (kTZ + 2 * P.hz) * sizeof(T);
+    const size_t smem = gamma_smem<T>(P.n_off, P.hx, P.hy, P.hz);
     int set = 0;                                // once per (device, kernel)
     PBD_TRY(smem_optin((const void*)gamma_kernel<T, false>, kGMaxSmem, 0, &set));
     PBD_TRY(smem_optin((const void*)gamma_kernel<T, true>, kGMaxSmem, 0, &set));
