@@ -179,11 +179,12 @@ fwd_f64_kernel(pbd_field f, const double* __restrict__ w, const double* __restri
     int l = next_active(0), j0 = 0, i0 = 0;
     if (l < f.n_layers) copy_w(l, 0, 0);
     double u[4][4];                    // U rows 16 m + g (+ 8), columns 8 warp + 2 t (+ 1)
-    // spot positions of a step's chunks, +inf (factor 0) past their ends
+    // spot positions of a step's chunks; past their ends any finite one, whose factors meet zero weights
+    // and zero rows of U (an infinite one gives NaN where a width's k2 underflows)
     auto stage_spots = [&](int j0, int i0) {
         const int q = tid & 63, n = (tid < 64 ? nsx - i0 : nsy - j0);
-        if (tid < 64) s_xs[q] = q < n ? f.x0 + ((double)(i0 + q) - cx) * f.dx_spot : INFINITY;
-        else if (tid < 128) s_ys[q] = q < n ? f.y0 + ((double)(j0 + q) - cy) * f.dy_spot : INFINITY;
+        if (tid < 64) s_xs[q] = q < n ? f.x0 + ((double)(i0 + q) - cx) * f.dx_spot : 0.0;
+        else if (tid < 128) s_ys[q] = q < n ? f.y0 + ((double)(j0 + q) - cy) * f.dy_spot : 0.0;
         __syncthreads();
     };
     stage_spots(0, 0);
@@ -243,9 +244,10 @@ fwd_f64_kernel(pbd_field f, const double* __restrict__ w, const double* __restri
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int j = 16 * m + 8 * h + g;
+                    const double sc = j < nj ? nrm : 0.0;        // an infinite nrm leaves the padding 0
                     if (j < pj)
                         *reinterpret_cast<double2*>(&U[j * kLDX + 8 * warp + 2 * t]) =
-                            make_double2(nrm * u[m][2 * h], nrm * u[m][2 * h + 1]);
+                            make_double2(sc * u[m][2 * h], sc * u[m][2 * h + 1]);
                 }
         }
         __syncthreads();
