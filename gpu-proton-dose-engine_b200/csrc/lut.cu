@@ -757,7 +757,11 @@ __global__ void __launch_bounds__(kMapThreads) wed_grad_maps_kernel(
             if (f & (1u << 30)) {
 #pragma unroll
                 for (int q = 0; q < kMapPer; ++q)
-                    if (in[q]) out[q][l * lstride] = (float)(curve_value(p[0][q], s_c[0][k].zmax, d[q]) * g[q]);
+                    if (in[q]) {             // 0 outside the curve, whatever the gradient there (inf, NaN)
+                        const double zm = s_c[0][k].zmax;
+                        const bool outside = d[q] < 0.0 || d[q] > zm;
+                        out[q][l * lstride] = outside ? 0.f : (float)(curve_value(p[0][q], zm, d[q]) * g[q]);
+                    }
             }
             if constexpr (kRange) {
                 if (f & (1u << 31)) {
