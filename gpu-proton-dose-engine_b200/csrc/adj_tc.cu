@@ -125,6 +125,7 @@ struct Params {
                          //    5 layers of 53 x 53 x 110 in a medium 76 us against 40, and
                          //    117 x 93 x 121 with 33 layers' adjoint 93 us against 86
     uint32_t o_b2, o_w, w_bytes, o_stage;   // shared-memory offsets: B, weights (two buffers), staging
+    float give_back;     // 2^-24: the split mode's results are raised by what truncation takes; else 0
     int sym;             // 1: every job is one tile and symmetric in x and y (grid, lattice, origins),
                          //    so B's rows equal the rows G evaluates for A
     int adapt;           // 1 (one job, no explicit schedule): every CTA counts the active pairs T
@@ -332,12 +333,6 @@ __device__ __forceinline__ void scheduler_warp(const Params& P, const Units U, S
                 st.bx = (float)((double)kOpScale * qx * qx);
                 const float ry = kBand * ivy, rx = kBand * ivx;
                 st.ry = ry; st.rx = rx;
-                // The tensor core truncates its FP32 accumulators: a result loses about 2^-24 of itself per
-                // k-step that matters to it.  Measured against 64 bits: 2.0e-7 (random dL/dD) to 2.4e-7 (of
-                // one sign, plan losses) at s = 2 voxels, 2.7e-7 to 4.1e-7 at 4.5 to 5, with a spread of
-                // 8e-8.  The plan losses' mean, 2^-24 (2 + 0.6 (s / dy + s / dx)), is given back here.
-                const double lost = (2.0 + 0.6 * (double)(ivy + ivx)) * 5.9604644775390625e-8;
-                st.nrm = (float)(kInv2Pi * is * is * (1.0 + lost));
                 st.inv_s = (float)is;
                 int e = 0;
                 (void)frexpf(1.001f + 2.50663f * ivy, &e);     // 1 + sqrt(2 pi) s / dy < 2^e
@@ -350,6 +345,16 @@ __device__ __forceinline__ void scheduler_warp(const Params& P, const Units U, S
                 // a band that misses the tile altogether: one group, of zeros
                 if (st.xa >= st.xb) { st.xa = 0; st.xb = 1; }
                 if (ya[0] >= yb[0] && ya[1] >= yb[1]) { ya[0] = 0; yb[0] = 1; }
+                // The tensor core truncates its FP32 accumulators: a result loses up to 1.2 x 2^-24 of itself
+                // per k-step (16-voxel group of the band) that matters to it, as many as the width spans.  Lost
+                // in units of 2^-24 on one tile, by width in voxels: a dL/dD of one sign 4 (2), 10 (5), 17 (10),
+                // 20 (14), 15 (100); of random sign 3, 4, 4, 4, 3; a single voxel 2 at any; over two row tiles one
+                // sign 10 (5), 16 (10), 28 (20), 33 (100).  Half-way between, no further than the band's own
+                // groups, is given back: 128 voxels or fewer stay within 1.2e-6 of the largest dL/dW at any
+                // width (0.5e-6 to 6 voxels), two row tiles within 2e-6.  Without it 1.8e-6 and 3.2e-6.
+                const float gy = (float)(yb[0] - ya[0] + yb[1] - ya[1]), gx = (float)(st.xb - st.xa);
+                const float lost = 2.0f + 0.6f * (fminf(ivy, 1.25f * gy) + fminf(ivx, 1.25f * gx));
+                st.nrm = (float)(kInv2Pi * is * is * (1.0 + (double)(lost * P.give_back)));
             }
             unsigned emit = __ballot_sync(FULL, mine);
             while (emit && ok) {
@@ -1149,6 +1154,7 @@ int launch_mode(const Params& P0, int max_nsy, cudaStream_t s) {
     int max_dyn = 0;
     PBD_TRY(smem_optin((const void*)adj_tc_kernel<kSplit>, -1, kLaunchRegsNeeded, &max_dyn));
     Params P = P0;
+    P.give_back = kSplit ? 5.9604644775390625e-8f : 0.f;
     const uint32_t narr = kSplit ? 2u : 1u;
     P.o_b2 = (uint32_t)P.tiles * narr * 128u * 128u * 2u;
     P.o_w = P.o_b2 + narr * 2u * (uint32_t)P.N1 * 128u * 2u;
