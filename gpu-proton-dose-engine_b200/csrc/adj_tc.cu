@@ -16,7 +16,7 @@
 // Precision.  Every split or TF32 mode runs split FP16: a = hi + lo, hi = fp16(a), lo = fp16(a - hi),
 // three products, FP32 accumulation; the BF16 mode runs plain BF16.  Operands are scaled by powers
 // of two into FP16's range, all exact: A and B by 2^14 (|s G'| <= 1), each unit's slice G so that
-// its largest value lands in [2^14, 2^15), and Y by 2^-(14 + ky), 2^ky >= 1 + sqrt(2 pi) s / dy,
+// its largest value lands in [2^14, 2^15), and Y by 2^-(14 + ky), 2^ky >= min(1 + sqrt(2 pi) s / dy, 256),
 // the bound on sum_y A.  Distances are formed in voxel units from the spot's integer and
 // fractional voxel position, so that a Gaussian's exponent is good to FP32 rounding of its own
 // size (from y0 + c dy - ys in FP32 the cancellation cost 1e-6 of it); the cross products go to the
@@ -335,8 +335,9 @@ __device__ __forceinline__ void scheduler_warp(const Params& P, const Units U, S
                 st.ry = ry; st.rx = rx;
                 st.inv_s = (float)is;
                 int e = 0;
-                (void)frexpf(1.001f + 2.50663f * ivy, &e);     // 1 + sqrt(2 pi) s / dy < 2^e
-                st.ky = e > 60 ? 60 : e;
+                // sum_y A < 1 + sqrt(2 pi) s / dy, and no more than the 256 rows, < 2^e
+                (void)frexpf(fminf(1.001f + 2.50663f * ivy, 256.5f), &e);
+                st.ky = e;
                 st.fy = __int_as_float((127 - 14 - st.ky) << 23);
                 band_groups(px0, px1, rx, J.nx, xt, st.xa, st.xb);
 #pragma unroll

@@ -66,3 +66,26 @@ def test_adjoint_at_any_width(shape, x0):
 
 def test_more_than_64_layers_on_several_tiles():
     _check(260, 140, 19, 23, tuple(0.5 * 1.35 ** k for k in range(15)), 0.02)       # 75 layers
+
+
+def test_widths_far_past_the_grid():
+    """Flat beams: Y's scale is bounded by the grid's rows, not by the width; no dose, no gradient in the limit."""
+    _check(64, 48, 17, 21, (1e4, 1e6, 1e9, 1e12), 0.02)
+    _check(150, 140, 17, 21, (1e4, 1e6, 1e9, 1e12), 0.02)
+
+
+@pytest.mark.parametrize("width", [1e45, 1e160, np.inf])
+def test_infinite_widths_give_zero(width):
+    import torch
+    pb = load_pkg()
+    rng = np.random.default_rng(0)
+    grid = pb.model.DoseGrid(40, 33, 2, VOX, VOX, VOX, -4.0, -3.0, 0.0)
+    lat = pb.model.SpotLattice(9, 7, 3, 0.25, 0.25, 0.0, 0.0, weights=rng.uniform(0.1, 1.0, (3, 7, 9)))
+    sig = np.full((3, 2), 0.4)
+    sig[1] = width
+    plan = pb.engines.DosePlan(pb.model.PBProblem(grid, lat, np.ones((3, 2)), sig), tables="problem")
+    g = torch.as_tensor(rng.uniform(-0.4, 1.0, grid.shape).astype(np.float32), device="cuda")
+    one = torch.ones(3, 2, dtype=torch.float64, device="cuda")
+    gw, gr = plan.adjoint(g, didd=one, dsig=one)
+    assert bool((gw[1] == 0).all()) and float(gr[1]) == 0.0
+    assert bool((gw[0] != 0).any()) and bool(torch.isfinite(gr).all())
