@@ -527,7 +527,7 @@ __device__ __forceinline__ void mma_warp(const Params& P, uint32_t sbase, uint32
 // ------------------------------------------------------------------------------------------
 // DR: a pair's Q (TMEM columns from tq: Q[., i] at 2 i, Q[., i'] at 2 i + 1) -> the pair's P slot and
 // this warp's share of the pair's two dot products.
-//  * Slot layout: P[j][i] = Q[j, i] scale, rows of n1 = nsx rounded up to 16 floats (columns i >= nsx
+//  * Slot layout: P[j][i] = Q[j, i] pow2 nrm, rows of n1 = nsx rounded up to 16 floats (columns i >= nsx
 //    hold 0), so that a j lane writes its 8 columns as two 16-byte stores.
 //  * A thread's columns: 8-column chunks c0 = 8 half + 16 t, so that both halves of a lane
 //    quadrant drain the same number of chunks.
@@ -538,7 +538,7 @@ __device__ __forceinline__ void mma_warp(const Params& P, uint32_t sbase, uint32
 // ------------------------------------------------------------------------------------------
 struct Prev {
     int nsx, nsy, pair;
-    float scale, inv_s;       // Q -> P; 1 / s
+    float pow2, nrm, inv_s;   // Q -> P: the operands' power of two, taken back first, then 1 / (2 pi s^2); 1 / s
     float *slot, *dot_p, *dot_s;
 };
 
@@ -555,6 +555,7 @@ __device__ __forceinline__ void drain_q(const Params& P, const Prev& pr, uint32_
     // a warp whose 32 rows are all padding (its first row 16 sp >= nsy) owns no entry: it skips
     // the TMEM loads and stores zero partials
     const bool pad = __shfl_sync(0xffffffffu, jrow, 0) >= pnsy;
+    const f32x2 p2 = pk(pr.pow2, pr.pow2);
     if (!pad) {
 #pragma unroll 1
         for (int c = 8 * half; c < n1; c += 16) {
@@ -567,10 +568,11 @@ __device__ __forceinline__ void drain_q(const Params& P, const Prev& pr, uint32_
             float pv[8];
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-                const float vi = __uint_as_float(r[2 * q]);
+                float vi, vd;          // the power of two comes off before W goes on: Q times W may overflow
+                upk(mul2(pk(__uint_as_float(r[2 * q]), __uint_as_float(r[2 * q + 1])), p2), vi, vd);
                 a0 = fmaf(vi, wv[q], a0);
-                a1 = fmaf(__uint_as_float(r[2 * q + 1]), wv[q], a1);
-                pv[q] = pr.scale * vi;
+                a1 = fmaf(vd, wv[q], a1);
+                pv[q] = pr.nrm * vi;
             }
             if (!deriv && row_ok) {
                 float4* o = reinterpret_cast<float4*>(slot_row + c);
@@ -584,8 +586,8 @@ __device__ __forceinline__ void drain_q(const Params& P, const Prev& pr, uint32_
     float v = deriv ? a0 + other : a0;
 #pragma unroll
     for (int o = 16; o > 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) pr.dot_p[warp] = pr.scale * v;
-    if (lane == 1) pr.dot_s[warp] = pr.scale * pr.inv_s * v;
+    if (lane == 0) pr.dot_p[warp] = pr.nrm * v;
+    if (lane == 1) pr.dot_s[warp] = pr.nrm * pr.inv_s * v;
 }
 
 // Symmetric fields: B's rows from A's (this lane's row m, read back from TMEM K chunk by K chunk;
@@ -708,7 +710,7 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
             int e = 0;
             (void)frexpf(__uint_as_float(mx), &e);        // the largest is below 2^e
             eg = (mx > 0u && finite) ? 15 - e : 0;        // and lands in [2^14, 2^15)
-            eg = eg > 110 ? 110 : eg;
+            eg = eg > 126 ? 126 : eg;
             const float gs = __int_as_float((127 + eg) << 23);
             const f32x2 gs2 = pk(gs, gs);
             // one column per thread, every other 8-row chunk
@@ -896,9 +898,9 @@ __device__ __forceinline__ void math_warps(const Params& P, uint8_t* smem, uint3
         // Q = 2^14 2^eg 2^-(14 + ky) 2^14 Q_true; a slice with a non-finite value gives NaN everywhere
         prev.nsx = nsx; prev.nsy = nsy; prev.pair = cur.pair;
         prev.slot = cur.slot; prev.dot_p = cur.dot_p; prev.dot_s = cur.dot_s;
-        prev.scale = finite ? cur.nrm * __int_as_float((127 + cur.ky - 14) << 23) *
-                                  __int_as_float((127 - eg) << 23)
-                            : __int_as_float(0x7fc00000);
+        const int ex = cur.ky - 14 - eg, e1 = max(ex, -100);       // [-139, 108]
+        prev.pow2 = __int_as_float((127 + e1) << 23);
+        prev.nrm = finite ? cur.nrm * __int_as_float((127 + ex - e1) << 23) : __int_as_float(0x7fc00000);
         prev.inv_s = cur.inv_s;
         have_prev = true;
         __syncwarp();
