@@ -52,10 +52,18 @@ def _store(d: dict) -> None:
         pass   # an unwritable cache only costs a re-tune
 
 
+def _tiled_adjoint(plan) -> bool:
+    """Whether the tensor-core adjoint serves a grid past one 128 x 128 tile.  Its items are layers;
+    such grids' adjoints once ran in FP32, whose items are depths."""
+    f = plan.field
+    return (plan.precision != _lib.PREC["fp32"] and max(f.nx, f.ny) > 128 and f.ny <= 256
+            and max(f.n_sx, f.n_sy) <= 64)
+
+
 def geometry_key(plan, op: str) -> str:
     f = plan.field
     return (f"{op}|{f.nx}x{f.ny}x{f.nz}|{f.n_sx}x{f.n_sy}x{f.n_layers}|p{plan.precision}"
-            f"|a{plan.active_pairs()}")
+            f"|a{plan.active_pairs()}" + ("|layers" if _tiled_adjoint(plan) else ""))
 
 
 @contextlib.contextmanager
@@ -69,9 +77,14 @@ def schedule(fwd: int, adj: int):
 
 
 def lookup(plan, op: str):
+    key = geometry_key(plan, op)
     with _lock:
-        v = _load().get(geometry_key(plan, op))
-    return tuple(v["schedule"]) if v else None
+        d = _load()
+    if key in d:
+        return tuple(d[key]["schedule"])
+    # an entry without the mark counts the adjoint's items in depths: only its forward holds
+    v = d.get(key.removesuffix("|layers"))
+    return (v["schedule"][0], 0) if v else None
 
 
 def tune(plan, op: str = "loss_grad", mask=None, presc=None, fwd_candidates=CANDIDATES_FWD,

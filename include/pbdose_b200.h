@@ -116,7 +116,8 @@ PBD_API int pbd_version(void);
 /* Validates a field descriptor; replaces pb_problem_validate, pencil_beam.cu:717-730. */
 PBD_API int pbd_field_validate(const pbd_field *f);
 /* Work-item granularity of the calling host thread's subsequent calls (0 = built-in
- * default): energy layers per forward item, depth slices per adjoint item.  The setting is
+ * default): energy layers per forward item; per adjoint item, layers on the tensor cores and
+ * depth slices in FP32.  The setting is
  * per host thread (calls from other threads keep their own), and the workspace queries use
  * it too, so set it before sizing.  No counterpart in the reference (it plays the role of
  * engines.torch_separable's layer_chunk knob). */
