@@ -847,59 +847,63 @@ __global__ void __launch_bounds__(kActThreads) wed_activity_kernel(const LayerSc
 // filling [z_i - dz/2, z_i + dz/2] with rho_i, water above the first voxel, path lengths
 // clipped at depth 0.  FP64.
 //
-// A block holds 32 columns and 16 runs of 8 depths (one per warp): each thread sums its run, the sums
-// of the runs above are added through shared memory, 128 depths at a time.  Bound by the latency of the
-// loads: one thread per column had 16 of them in flight in 4 warps per SM (128^3: 31 us), now 8 in
-// 32 warps (12 us).
-constexpr int kRayCols = 32, kRayRuns = 16, kRayLen = 8;
+// A block holds 32 columns and kRuns runs of 8 depths (one per warp): each thread sums its run, the sums
+// of the runs above are added through shared memory, 8 kRuns depths at a time; the path lengths, the
+// same for every column, come from a table of the pass.  Few columns are bound by the latency of the loads (one
+// thread per column, 16 in flight: 128^3 17.8 us, now 6.9), many by FP64 issue, which the sums of the runs
+// and warps without a depth of their own add to.  So as many runs as the depths fill, up to 16 below 16,000 columns,
+// 4 below 100,000 and 1 (a thread per column) above; the sums' order is the same for any number.  Sixteen for
+// every grid, path lengths in each thread, against one thread per column before that and now: 512 x 512 x 64
+// 121, 50, 40 us; 512 x 512 x 150 237, 114, 91; 128 x 128 x 1 7.3, 2.3, 2.5; 200 x 200 x 256 48, 68, 35.
+constexpr int kRayCols = 32, kRayLen = 8, kRayMaxRuns = 16;
 
-__global__ void __launch_bounds__(kRayCols * kRayRuns, 2) wed_raytrace_kernel(int nz, size_t ncol, double oz,
-                                                                           double dz,
-                                                                           const float* __restrict__ rho,
-                                                                           double* __restrict__ wed) {
-    __shared__ double sums[2][kRayRuns][kRayCols];
+template <int kRuns>
+__global__ void __launch_bounds__(kRayCols * kRuns, 32 / kRuns) wed_raytrace_kernel(
+    int nz, size_t ncol, double oz, double dz, const float* __restrict__ rho, double* __restrict__ wed) {
+    __shared__ double sums[2][kRuns][kRayCols];
+    __shared__ double2 s_len[2][kRuns * kRayLen];        // path to each depth's voxel centre and through the voxel
     const int lane = threadIdx.x & 31, run = threadIdx.x >> 5;
-    auto depths = [&](int k, double& lo, double& mid, double& hi) {
-        const double zc = oz + (double)k * dz;
-        lo = fmax(zc - 0.5 * dz, 0.0);
-        mid = fmax(zc, 0.0);
-        hi = fmax(zc + 0.5 * dz, 0.0);
-    };
     int buf = 0;
     for (size_t c0 = (size_t)blockIdx.x * kRayCols; c0 < ncol; c0 += (size_t)gridDim.x * kRayCols) {
         const size_t c = c0 + lane;
         const bool in = c < ncol;
         double above = fmax(oz - 0.5 * dz, 0.0);         // water above the first voxel
-        for (int k0 = 0; k0 < nz; k0 += kRayRuns * kRayLen) {
+        for (int k0 = 0; k0 < nz; k0 += kRuns * kRayLen) {
             const int kr = k0 + run * kRayLen;
             float r[kRayLen];
 #pragma unroll
             for (int q = 0; q < kRayLen; ++q)
                 r[q] = in && kr + q < nz ? __ldcs(rho + (size_t)(kr + q) * ncol + c) : 0.f;
-            double sum = 0.0;
-#pragma unroll
-            for (int q = 0; q < kRayLen; ++q) {
-                double lo, mid, hi;
-                depths(kr + q, lo, mid, hi);
-                sum += (double)r[q] * (hi - lo);
+            if (threadIdx.x < kRuns * kRayLen) {
+                const double zc = oz + (double)(k0 + (int)threadIdx.x) * dz;
+                const double lo = fmax(zc - 0.5 * dz, 0.0), mid = fmax(zc, 0.0), hi = fmax(zc + 0.5 * dz, 0.0);
+                s_len[buf][threadIdx.x] = make_double2(mid - lo, hi - lo);
             }
-            sums[buf][run][lane] = sum;
             __syncthreads();
+            const double2* len = s_len[buf] + run * kRayLen;
             double acc = above;
+            if constexpr (kRuns > 1) {
+                double sum = 0.0;
+#pragma unroll
+                for (int q = 0; q < kRayLen; ++q) sum += (double)r[q] * len[q].y;
+                sums[buf][run][lane] = sum;
+                __syncthreads();
 #pragma unroll 4
-            for (int w = 0; w < kRayRuns; ++w) {
-                if (w == run) acc = above;
-                above += sums[buf][w][lane];
+                for (int w = 0; w < kRuns; ++w) {
+                    if (w == run) acc = above;
+                    above += sums[buf][w][lane];
+                }
             }
-            buf ^= 1;                                    // the next pass's sums: no barrier here
+            double own = 0.0;
 #pragma unroll
             for (int q = 0; q < kRayLen; ++q) {
-                double lo, mid, hi;
-                depths(kr + q, lo, mid, hi);
                 const double rr = (double)r[q];
-                if (in && kr + q < nz) __stcs(wed + (size_t)(kr + q) * ncol + c, acc + rr * (mid - lo));
-                acc += rr * (hi - lo);
+                if (in && kr + q < nz) __stcs(wed + (size_t)(kr + q) * ncol + c, acc + rr * len[q].x);
+                acc += rr * len[q].y;
+                if (kRuns == 1) own += rr * len[q].y;
             }
+            if (kRuns == 1) above += own;
+            buf ^= 1;                                    // the next pass's tables: no barrier here
         }
     }
 }
@@ -1208,7 +1212,17 @@ int lut_wed_raytrace(int nz, int ny, int nx, double oz, double dz, const float* 
     if (!isfinite(oz) || !(dz > 0.0) || !isfinite(dz)) return PBD_ERR_BAD_VALUE;
     const size_t ncol = (size_t)ny * nx;
     const int blocks = (int)std::min<size_t>((ncol + kRayCols - 1) / kRayCols, (size_t)num_sms() * 32);
-    wed_raytrace_kernel<<<blocks, kRayCols * kRayRuns, 0, st>>>(nz, ncol, oz, dz, rho, wed);
+    // the least power of two of runs that holds every depth; 4 at most from 16,000 columns on, 1 from 100,000
+    // (256 x 256 x 128: 4 runs 20 us, 1 25, 16 27; 350 x 350 x 100: 1 run 32, 4 38; 64 x 64 x 256: 16 runs 4.8, 4 8.6)
+    const int most = ncol >= 100000 ? 1 : ncol >= 16000 ? 4 : kRayMaxRuns;
+    int runs = 1;
+    while (runs < most && runs * kRayLen < nz) runs *= 2;
+    const auto kernel = runs == 1   ? wed_raytrace_kernel<1>
+                        : runs == 2 ? wed_raytrace_kernel<2>
+                        : runs == 4 ? wed_raytrace_kernel<4>
+                        : runs == 8 ? wed_raytrace_kernel<8>
+                                    : wed_raytrace_kernel<kRayMaxRuns>;
+    kernel<<<blocks, kRayCols * runs, 0, st>>>(nz, ncol, oz, dz, rho, wed);
     PBD_LAUNCH_CHECK();
     count_launch(1);
     return PBD_OK;
