@@ -480,7 +480,10 @@ lut_eval_kernel(pbd_lut_spec spec, LutDims dm, const LayerScal* __restrict__ sca
                 const double* __restrict__ smooth, const double* __restrict__ t_fe,
                 double single_depth, double* idd, double* sigma, double* didd, double* dsig) {
     __shared__ double s_i[3][kEvalDepths], s_s[3][kEvalDepths];
-    asm volatile("griddepcontrol.wait;" ::: "memory");   // the arrays of this call
+    // The arrays of this call.  They are read through L1's read-only path below (__ldg), which may hold only
+    // what was complete when this grid started: so the kernels before it must not trigger its launch
+    // (griddepcontrol.launch_dependents), and do not -- it starts as their blocks end.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int nb = (dm.nz + kEvalDepths - 1) / kEvalDepths;      // blocks per layer
     const int l = blockIdx.x / nb, k0 = (blockIdx.x - l * nb) * kEvalDepths;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
