@@ -242,7 +242,7 @@ class DosePlan:
         return out
 
     def forward_f64(self, w=None, out=None):
-        """The dose in FP64 on the CUDA cores (pbd_forward_f64): weights, Gaussians, products
+        """The dose in FP64 (pbd_forward_f64): weights, Gaussians, products
         and sums in float64.  ``w`` defaults to the plan's weights (float32 values, exact in
         float64); returns a float64 (nz, ny, nx) tensor."""
         torch = self.torch
@@ -271,6 +271,11 @@ class DosePlan:
     # -- adjoint -------------------------------------------------------------------
     def adjoint(self, grad_dose, w=None, idd=None, sigma=None, didd=None, dsig=None,
                 with_range: bool = True):
+        """(dL/dW, dL/dR) for a dL/dD of the caller's (``pbd_adjoint``); dL/dR is None without the
+        derivative tables.  The split-FP16 modes scale dL/dD by the largest value of a slice's 128
+        columns and keep 39 bits below it (22 of the value itself down to 2^-17 of the largest), and
+        hold an FP32 map per (layer, slice, 128 columns) as scratch; ``precision="fp32"`` has
+        neither limit."""
         torch = self.torch
         w = self._weights(w)
         idd = self.idd if idd is None else idd
@@ -466,7 +471,7 @@ def torch_separable(problem, device: str = "cuda", dtype=None, allow_tf32: bool 
     * ``dtype``: None or torch.float32 give a float32 dose from the tensor cores (split
       FP16, three products with power-of-two scaling: within 1e-6 of FP64; lattices wider
       than 64 spots use the FP32 kernel on the CUDA cores); torch.float64 gives a float64
-      dose computed in FP64 on the CUDA cores (the reference's float64 mode, ~1e-15).
+      dose computed in FP64 (the reference's float64 mode, ~1e-15).
     * ``allow_tf32``: the reference's flag for TF32 tensor cores; its run with the flag
       kept FP32 accuracy (1.51e-7, benchmark_full.json:68-81), so it keeps the default
       split form, within 1e-6.  One-product TF32 (~1e-4) is available only as

@@ -53,7 +53,10 @@ def wed_raytrace(rho, grid, device=None):
 class WedPlan:
     """One field in a heterogeneous medium: the lateral widths of water at the geometric
     depths and the layers' depth curves (``pbd_build_wed_curves``), built once on the device,
-    and the workspaces of ``pbd_forward_wed_curves`` and (on first use) ``pbd_adjoint_wed``."""
+    and the workspaces of ``pbd_forward_wed_curves`` and (on first use) ``pbd_adjoint_wed``.
+
+    ``precision``: "tf32x3" and "fp16x3" both take the split-FP16 kernels, whose weights are
+    scaled by their layer's largest (22 bits down to 2^-17 of it); "fp32" is FP32 throughout."""
 
     def __init__(self, problem, *, precision: str = "tf32x3", device=None,
                  idd_model: ph.IDDModel = ph.DEFAULT_IDD, sigma_x0: float = 0.30,

@@ -55,13 +55,20 @@ extern "C" {
 /* Arithmetic used for the two Gaussian contractions.  All accumulate in FP32. */
 #define PBD_PREC_FP32    0   /* FP32 FMA on the CUDA cores */
 #define PBD_PREC_TF32X3  1   /* tcgen05 TF32, hi/lo split, three products (the lateral maps of a
-                                dose in a medium: as FP16X3, which is nearer to 64 bits) */
+                                dose in a medium: as FP16X3, which is nearer to 64 bits for weights
+                                within 2^-17 of their layer's largest) */
 #define PBD_PREC_TF32    2   /* tcgen05 TF32, one product */
 #define PBD_PREC_BF16X3  3   /* tcgen05 BF16, hi/lo split, three products */
 #define PBD_PREC_BF16    4   /* tcgen05 BF16, one product */
 #define PBD_PREC_FP16X3  5   /* tcgen05 FP16, hi/lo split, three products; operands scaled by
                                 powers of two into FP16's range.  The adjoint of every mode but
-                                FP32 and BF16 */
+                                FP32 and, up to 128 x 128 voxels, BF16 */
+
+/* Range of the FP16X3 operands.  A layer's weights are scaled by its largest, a slice's dL/dD by the largest
+ * of its 128 columns, Gaussians by their peak: 22 bits down to 2^-17 of that, then 39 bits below it (a value of
+ * 2^-23 of the largest keeps 16 bits, of 2^-30 nine).  Gaussians end at 8 widths in the adjoint.  So a voxel
+ * or spot that only weights, dL/dD or tails far below the largest reach is good to about 2^-38 of what the largest
+ * would give it, not to 22 bits of itself; where that matters, ask for PBD_PREC_FP32. */
 
 #define PBD_MAX_JOBS 128     /* jobs (fields x scenarios) per batched launch */
 
@@ -174,9 +181,9 @@ PBD_API int pbd_forward(const pbd_field *f, const float *w, const double *idd, c
 /* ---- forward dose in FP64 ----------------------------------------------------------
  * Replaces engines.torch_separable(..., dtype=torch.float64) on CUDA, engines.py:223-224 and
  * 230-274 (operands and both batched matmuls in float64).  The dose of pbd_forward with the
- * weights, Gaussians, products and sums in float64 on the CUDA cores: w (L, nsy, nsx) and
- * dose (nz, ny, nx) are float64.  No workspace: one block per (64 x 64 voxel tile, slice) sums
- * every layer in layer order and writes its voxels once. */
+ * weights, Gaussians, products and sums in float64 (FP64 matrix instructions): w (L, nsy, nsx)
+ * and dose (nz, ny, nx) are float64.  No workspace: one block per (tile of 64 columns and 64 or 128
+ * rows, slice) sums every layer in layer order and writes its voxels once. */
 PBD_API int pbd_forward_f64(const pbd_field *f, const double *w, const double *idd,
                             const double *sigma, double *dose, void *stream);
 
@@ -199,7 +206,14 @@ PBD_API int pbd_forward_noalloc(const pbd_field *f, const float *w, const double
 /* ---- adjoint (no counterpart in the reference, which has no gradient) --------------
  * Given grad_dose = dL/dD (nz, ny, nx), writes grad_w = dL/dW (L, nsy, nsx) and
  * grad_range = dL/d(range shift) (L), the latter through didd_dr and dsigma_dr
- * (either may be NULL together with grad_range == NULL to skip it). */
+ * (either may be NULL together with grad_range == NULL to skip it).
+ * In every precision but FP32 the tensor cores take lattices of up to 64 x 64 spots on grids of up to 256 rows
+ * and any number of columns (media: 128 x 128); other fields run in FP32 (batched loss gradients refuse what
+ * the tensor cores do not take, past 128 x 128 voxels among it).  Past 128 x 128
+ * voxels the BF16 mode's adjoint is FP16X3, as it was FP32 before.  Its workspace holds one map of n_sy *
+ * (n_sx rounded up to 16) floats per (layer, slice, 128 columns), reached or not: 482 MB for 200 x 200 x 256 and 60
+ * layers of 61 x 61 spots, where the FP32 adjoint takes 57 MB.  Past 128 x 128 voxels a field that would take
+ * more than 8 GiB runs in FP32; PBD_PREC_FP32 keeps the small workspace for any. */
 PBD_API int pbd_adjoint_workspace(const pbd_field *f, int precision, size_t *bytes);
 PBD_API int pbd_adjoint(const pbd_field *f, const float *w, const double *idd, const double *sigma,
                 const double *didd_dr, const double *dsigma_dr, const float *grad_dose,
