@@ -26,19 +26,21 @@ constexpr int SC = kSpotChunk;                      // 64 spots per chunk
 constexpr size_t fwd_smem(int ry, int rx, int scx, int scy) {
     return (size_t)(16 * (rx * scx + (rx + ry) * scy) + scx * SC) * sizeof(float);
 }
-// Spots per chunk of an axis of n: equal parts of at most 64, in fours (73 spots as 40 + 33, not 64 + 9).
-// Each axis of each job has its own.  One size for the launch, from its widest axis, cut 41 spots beside
-// 73 into 40 + 1, each part with its own weights, factors and barriers: 128 x 128 x 64, 73 x 41 spots,
-// 10 layers 302 us, now 217; a batch of three 41 x 41 fields and a small one of 73 x 73 386, now 306.
-__host__ __device__ constexpr int spot_chunk(int n) {
-    const int parts = (n + SC - 1) / SC;
-    return ((n + parts - 1) / parts + 3) / 4 * 4;
+// Spots per chunk of an axis of n: equal parts of at most 64, in fours along x (73 spots as 40 + 33, not 64 + 9).
+// Along y, where U's rows come in groups of 16, a cut lies on a group (69 spots as 48 + 21, 80 rows, not 36 + 33,
+// 96: 150 x 142 x 130, 73 x 69 spots, 24 layers on every slice 1208 us, now 1171).  Each axis of each job has its
+// own.  One size for the launch, from its widest axis, cut 41 spots beside 73 into 40 + 1, each part with its
+// own weights, factors and barriers: 128 x 128 x 64, 73 x 41 spots, 10 layers 302 us, now 217; a batch of three
+// 41 x 41 fields and a small one of 73 x 73 386, now 306.
+__host__ __device__ constexpr int spot_chunk(int n, int group = 4) {
+    const int parts = (n + SC - 1) / SC, g = parts > 1 ? group : 4;
+    return ((n + parts - 1) / parts + g - 1) / g * g;
 }
 
 // Tile sizes per axis, in units of 16 voxels.  An axis of n voxels is cut into ceil(n / 128) tiles of
 // equal size, rounded up to one of these: a 150 x 142 slice in four 80 x 80 tiles instead of four
 // 128 x 128 ones, of which two thirds were outside the grid.  The kernel is bound by FP32 FMA issue, so
-// its time follows the padded area: 150 x 142 x 130, 24 layers of 73 x 69 spots (cut in chunks of 40 and 36
+// its time follows the padded area: 150 x 142 x 130, 24 layers of 73 x 69 spots (cut in chunks of 40 and 48
 // for the same reason, where 64 + 9 were padded to 128): 1143 us with 128 x 128 tiles and 64-spot chunks, 640
 // with these, 605-626 with three blocks to an SM (which small tiles allow and large ones do not: an
 // 8 x 8 register tile needs 128 registers).  A grid of 128 keeps its 128 x 128 tile: two of 64 x 128
@@ -222,7 +224,7 @@ fwd_simt_kernel(const JobDev* __restrict__ jobs, const FwdItem* __restrict__ ite
         const JobDev& J = jobs[it.job];
         const int nz = J.nz, nx = J.nx, ny = J.ny, nsx = J.nsx, nsy = J.nsy;
         const int z = it.z, y0 = it.ty * TY, x0 = it.tx * TX;
-        const int scx = spot_chunk(nsx), scy = spot_chunk(nsy);
+        const int scx = spot_chunk(nsx), scy = spot_chunk(nsy, 16);
         const bool chunks = scx < nsx || scy < nsy;
         // the chunk's spot positions: once per item where the lattice is one chunk
         auto stage_spots = [&](int j0, int i0) {
@@ -435,7 +437,7 @@ int launch_forward(JobDev* jobs_dev, const JobDev* jobs_host, int n_jobs, FwdIte
     int mx = 4, my = 4;
     for (int j = 0; j < n_jobs; ++j) {
         mx = std::max(mx, spot_chunk(jobs_host[j].nsx));
-        my = std::max(my, spot_chunk(jobs_host[j].nsy));
+        my = std::max(my, spot_chunk(jobs_host[j].nsy, 16));
     }
     const FwdKernel kernel = pick_kernel(ry, rx);
     PBD_TRY(smem_optin((const void*)kernel, (int)fwd_smem(ry, rx, SC, SC), 0, &set));
