@@ -51,8 +51,8 @@
 // 510, waits for the MMAs 800 of 5500 on the 128^3 / 41 x 41 x 40 field), not the tensor pipe.
 // Straight-line code is fetched anew for every pair at some 10 cycles an instruction, so every
 // phase is a rolled loop over 16-column groups: unrolled, with fewer instructions executed, the same
-// phases took 7800 cycles.  The adjoint of that field: 85 us before (split BF16 with two columns per
-// 27 instructions, unrolled, whole tiles, weights loaded by the math warps), 64 us now, and 20 of its
+// phases took 7800 cycles.  The adjoint of that field: 90 us before (split BF16 with two columns per
+// 27 instructions, unrolled, whole tiles, weights loaded by the math warps), 71 us now, and 20 of its
 // gradients' jobs in four fields 1413 -> 990 us; a 200 x 200 x 256 field's (which ran in FP32 on the
 // CUDA cores) 12.4 -> 0.83 ms.
 //
