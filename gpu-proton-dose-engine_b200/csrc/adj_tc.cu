@@ -352,7 +352,7 @@ __device__ __forceinline__ void scheduler_warp(const Params& P, const Units U, S
                 // 20 (14), 15 (100); of random sign 3, 4, 4, 4, 3; a single voxel 2 at any; over two row tiles one
                 // sign 10 (5), 16 (10), 28 (20), 33 (100).  Half-way between, no further than the band's own
                 // groups, is given back: 128 voxels or fewer stay within 1.2e-6 of the largest dL/dW at any
-                // width (0.5e-6 to 6 voxels), two row tiles within 2e-6.  Without it 1.8e-6 and 3.2e-6.
+                // width (0.6e-6 to 6 voxels), two row tiles within 2.1e-6.  Without it 1.8e-6 and 3.2e-6.
                 const float gy = (float)(yb[0] - ya[0] + yb[1] - ya[1]), gx = (float)(st.xb - st.xa);
                 const float lost = 2.0f + 0.6f * (fminf(ivy, 1.25f * gy) + fminf(ivx, 1.25f * gx));
                 st.nrm = (float)(kInv2Pi * is * is * (1.0 + (double)(lost * P.give_back)));
